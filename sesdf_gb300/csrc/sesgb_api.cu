@@ -882,11 +882,18 @@ extern "C"
     }
 
     // ---- signed distance at query points ---------------------------------------
-    static int sdf_prepare( sesgb_ctx * c, uint32_t m, cudaStream_t s )
+    static int sdf_prepare( sesgb_ctx * c, uint32_t m, SdfState & st, cudaStream_t s )
     {
         if ( !c->built )
             return SESGB_ERR_NOT_BUILT;
-        const size_t need = sdf_scratch_bytes( m );
+        if ( c->mode != SESGB_MODE_FULL || c->nMol != 1 )
+        {
+            c->err = "the SDF needs a full-surface build of one molecule";
+            return SESGB_ERR_MODE;
+        }
+        st.rmax           = c->hCounts->rmax;
+        st.general        = c->hCounts->nbrTruncated > 0 || c->hCounts->outside > 0;
+        const size_t need = sdf_scratch_bytes( c->b, st, m );
         if ( need > c->sdfScratchBytes )
         {
             if ( c->sdfScratch )
@@ -902,15 +909,7 @@ extern "C"
             }
             c->sdfScratchBytes = need;
         }
-        if ( c->mode != SESGB_MODE_FULL || c->nMol != 1 )
-        {
-            c->err = "the SDF needs a full-surface build of one molecule";
-            return SESGB_ERR_MODE;
-        }
-        const float reach = c->hCounts->rmax + 2.f * c->rp + SESGB_SDF_BAND;
-        launch_fine_params( c->b, reach, c->n, s );
-        launch_cells( c->b, 2, c->n, nullptr, c->scanScratch, s );
-        return cuda_ok( c, cudaGetLastError(), "sdf grid" ) ? SESGB_OK : SESGB_ERR_CUDA;
+        return SESGB_OK;
     }
 
     int sesgb_sdf( sesgb_ctx * c, const float * device_queries, uint32_t m, float * device_sdf, int * device_kind, void * stream )
@@ -918,10 +917,11 @@ extern "C"
         if ( !c || ( m && ( !device_queries || !device_sdf ) ) )
             return SESGB_ERR_INVALID;
         cudaStream_t s  = static_cast<cudaStream_t>( stream );
-        int          st = sdf_prepare( c, m, s );
+        SdfState     q;
+        int          st = sdf_prepare( c, m, q, s );
         if ( st != SESGB_OK )
             return st;
-        launch_sdf( c->b, device_queries, m, SESGB_SDF_BAND, device_sdf, device_kind, c->sdfScratch, s );
+        launch_sdf( c->b, q, device_queries, m, SESGB_SDF_BAND, device_sdf, device_kind, c->sdfScratch, s );
         return cuda_ok( c, cudaGetLastError(), "sdf" ) ? SESGB_OK : SESGB_ERR_CUDA;
     }
 
@@ -931,12 +931,13 @@ extern "C"
         if ( !c || !device_grad_atoms || ( m && ( !device_queries || !device_grad_sdf ) ) )
             return SESGB_ERR_INVALID;
         cudaStream_t s  = static_cast<cudaStream_t>( stream );
-        int          st = sdf_prepare( c, m, s );
+        SdfState     q;
+        int          st = sdf_prepare( c, m, q, s );
         if ( st != SESGB_OK )
             return st;
         if ( !c->gradSorted && !cuda_ok( c, cudaMalloc( &c->gradSorted, sizeof( float ) * 4 * std::max<size_t>( c->n, 1 ) ), "cudaMalloc" ) )
             return SESGB_ERR_CUDA;
-        launch_sdf_backward( c->b, device_queries, m, SESGB_SDF_BAND, device_grad_sdf, c->gradSorted, device_grad_atoms,
+        launch_sdf_backward( c->b, q, device_queries, m, SESGB_SDF_BAND, device_grad_sdf, c->gradSorted, device_grad_atoms,
                              c->sdfScratch, s );
         return cuda_ok( c, cudaGetLastError(), "sdf backward" ) ? SESGB_OK : SESGB_ERR_CUDA;
     }
@@ -947,7 +948,8 @@ extern "C"
              || cam->max_steps > ( 1u << 20 ) || !( cam->eps > 0.0 ) || !( cam->normal_step > 0.0 ) )
             return SESGB_ERR_INVALID;
         cudaStream_t s  = static_cast<cudaStream_t>( stream );
-        int          st = sdf_prepare( c, 0, s );
+        SdfState     q;
+        int          st = sdf_prepare( c, 0, q, s );
         if ( st != SESGB_OK )
             return st;
         TraceParams p;
@@ -966,7 +968,7 @@ extern "C"
         p.width      = cam->width;
         p.height     = cam->height;
         p.maxSteps   = cam->max_steps;
-        launch_trace( c->b, p, SESGB_SDF_BAND, device_depth, device_normals, s );
+        launch_trace( c->b, q, p, SESGB_SDF_BAND, device_depth, device_normals, c->sdfScratch, s );
         return cuda_ok( c, cudaGetLastError(), "render" ) ? SESGB_OK : SESGB_ERR_CUDA;
     }
 

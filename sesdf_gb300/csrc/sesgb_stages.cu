@@ -13,7 +13,6 @@
 //   k_segment_counts/k_segments      buildConicPatches + buildSegments (operations.inl:488-668)
 //   k_probe_neighbors        handleIntersectionSingularities + findIntersectionsNeighbors (operations.cu:14-32,271-338)
 //   k_tori_count/k_tori      fillCircles (ssesdf/operations.cu:246-285)
-//   k_sdf                    signed distance at query points and its adjoint (no reference counterpart)
 //
 // Every predicate is first evaluated in float32 in coordinates relative to the
 // owning atom; when its margin is inside a conservative band (kRel times the
@@ -24,29 +23,13 @@
 #include <atomic>
 #include <cfloat>
 
+#include "sesgb_grid.cuh"
 #include "sesgb_stages.cuh"
 
 namespace sesgb
 {
     namespace
     {
-        constexpr float kRel = 1.0f / 65536.0f;
-
-        __device__ __forceinline__ int3 fine_cell( const FineGrid & g, float x, float y, float z )
-        {
-            int cx = (int)floorf( ( x - g.origin.x ) / g.h );
-            int cy = (int)floorf( ( y - g.origin.y ) / g.h );
-            int cz = (int)floorf( ( z - g.origin.z ) / g.h );
-            cx     = cx < 0 ? 0 : ( cx >= g.dims.x ? g.dims.x - 1 : cx );
-            cy     = cy < 0 ? 0 : ( cy >= g.dims.y ? g.dims.y - 1 : cy );
-            cz     = cz < 0 ? 0 : ( cz >= g.dims.z ? g.dims.z - 1 : cz );
-            return make_int3( cx, cy, cz );
-        }
-        __device__ __forceinline__ uint32_t fine_key( const FineGrid & g, int3 c )
-        {
-            return ( (uint32_t)c.z * (uint32_t)g.dims.y + (uint32_t)c.y ) * (uint32_t)g.dims.x + (uint32_t)c.x;
-        }
-
         // The 27 cells around c as 9 rows of up to three x-adjacent cells, each a
         // contiguous range of the cell-ordered item array. Lane r < 9 computes row r;
         // every lane receives all nine (start, exclusive prefix) pairs.
@@ -274,14 +257,10 @@ namespace sesgb
         {
             float4   p;
             uint32_t m = 0;
-            if ( kind == 0 || kind == 2 )
+            if ( kind == 0 )
             {
                 p = b.atoms[ q ];
                 m = mol_of( b, q );
-                // kind 2 (SDF queries): the sign of the radius marks an atom without any
-                // accessible surface (neighbours present, every circle buried)
-                if ( kind == 2 && b.visCnt[ q ] == 0 && b.nbrCount[ q ] > 0 )
-                    p.w = -p.w;
             }
             else
             {
@@ -338,67 +317,6 @@ namespace sesgb
         {
             const d3 dd = dsub( D3( pq ), D3( pp ) );
             return __dsqrt_rn( ddot( dd, dd ) ) < 2.0 * (double)rp;
-        }
-
-        // The 25 rows of a span-2 stencil (cells of at least half the largest pair cutoff) around
-        // atom position p, each cut to the x-range that can hold a neighbour of the atom: a
-        // neighbour j lies within cut = R_i + R_max (+ margins) of p, so a row (y, z) whose cells
-        // keep |dy|, |dz| >= ey, ez from p only needs x within sqrt(cut^2 - ey^2 - ez^2) of p.
-        // Lane r < 25 computes row r; the rows' first items and exclusive prefixes go to shared
-        // memory (start[25], pre[26] with pre[25] = total), and the total is returned. A cell two
-        // beyond the atom's own along any axis starts at least 2h >= the largest pair cutoff away.
-        __device__ __forceinline__ uint32_t stencil_rows_span2( const FineGrid & g, const uint32_t * cellStart, float4 p,
-                                                                float cut, uint32_t * start, uint32_t * pre )
-        {
-            const uint32_t lane = lane_id();
-            const int3     c    = fine_cell( g, p.x, p.y, p.z );
-            uint32_t       st = 0, len = 0;
-            if ( lane < 25u )
-            {
-                const int y = c.y + (int)( lane % 5u ) - 2;
-                const int z = c.z + (int)( lane / 5u ) - 2;
-                if ( y >= 0 && z >= 0 && y < g.dims.y && z < g.dims.z )
-                {
-                    const float ylo = g.origin.y + (float)y * g.h, zlo = g.origin.z + (float)z * g.h;
-                    const float ey  = fmaxf( 0.f, fmaxf( ylo - p.y, p.y - ( ylo + g.h ) ) );
-                    const float ez  = fmaxf( 0.f, fmaxf( zlo - p.z, p.z - ( zlo + g.h ) ) );
-                    const float w2  = cut * cut - ey * ey - ez * ez;
-                    if ( w2 >= 0.f )
-                    {
-                        const float w  = sqrtf( w2 ) + 0.01f;
-                        int         x0 = (int)floorf( ( p.x - w - g.origin.x ) / g.h );
-                        int         x1 = (int)floorf( ( p.x + w - g.origin.x ) / g.h );
-                        x0             = max( x0, max( c.x - 2, 0 ) );
-                        x1             = min( x1, min( c.x + 2, g.dims.x - 1 ) );
-                        if ( x0 <= x1 )
-                        {
-                            st  = cellStart[ fine_key( g, make_int3( x0, y, z ) ) ];
-                            len = cellStart[ fine_key( g, make_int3( x1, y, z ) ) + 1 ] - st;
-                        }
-                    }
-                }
-            }
-            uint32_t       total;
-            const uint32_t ex = warp_exclusive_sum( len, total );
-            if ( lane < 25u )
-            {
-                start[ lane ] = st;
-                pre[ lane ]   = ex;
-            }
-            if ( lane == 0 )
-                pre[ 25 ] = total;
-            __syncwarp();
-            return total;
-        }
-        // cell-item index of stencil item f (f < total): the last row whose prefix is <= f
-        __device__ __forceinline__ uint32_t row_item_span2( const uint32_t * start, const uint32_t * pre, uint32_t f )
-        {
-            uint32_t r = 0;
-#pragma unroll
-            for ( uint32_t step = 16; step > 0; step >>= 1 )
-                if ( r + step < 25u && pre[ r + step ] <= f )
-                    r += step;
-            return start[ r ] + ( f - pre[ r ] );
         }
 
         template<int W>
@@ -3088,848 +3006,5 @@ namespace sesgb
         const uint64_t total = (uint64_t)b.n * b.cap + 1;
         k_reference_fill<<<min( persistent_blocks( 256 ), blocks_for( total, 256 ) ), 256, 0, s>>>( b, globalToTrimmed );
         counted();
-    }
-} // namespace sesgb
-
-// ---- signed distance to the SES at query points -----------------------------
-//
-// Definition (project-written; the reference has no SDF). E is the set of
-// probe-centre positions that overlap no atom: outside every SAS sphere
-// (radius R_i = r_i + rp). With T = rp + kSdfBand:
-//   x outside the SAS:  sdf = min_i (|x - c_i| - r_i), clamped to kSdfBand;
-//   x inside the SAS:   sdf = rp - min(T, dist(x, dE)).
-// dE is the SAS surface: the accessible parts of the SAS spheres, the arcs of
-// the visible circles and the probe positions. The nearest point of dE is the
-// radial projection of x on a sphere, the nearest point of a circle, or a
-// probe, whichever is nearest among those that lie on dE (not strictly inside
-// another SAS sphere); only atoms with |x - c_i| <= R_i + T can carry one.
-// The gradient with respect to the atoms follows the active primitive: the
-// sphere or atom distance directly, a circle point and a probe by the
-// Lagrange / implicit-function rule for points constrained to |p - c_m| = R_m.
-namespace sesgb
-{
-    namespace
-    {
-        constexpr int   kSdfWarps = 4;   // warps per block (one query per warp)
-        constexpr int   kSdfList   = 256; // atoms within reach held per query
-        constexpr int   kSdfStaged = 128; // neighbour slots staged in shared memory
-
-        enum SdfKind : int
-        {
-            kSdfClampInside = 0, // deeper than T below dE
-            kSdfAtom        = 1, // outside the SAS: nearest vdW sphere
-            kSdfClampOutside = 2,
-            kSdfSphere      = 3, // radial projection on an accessible SAS sphere patch
-            kSdfCircle      = 4, // nearest point of an accessible arc
-            kSdfProbe       = 5, // probe position (vertex of dE)
-        };
-
-        struct SdfHit
-        {
-            int    kind;
-            int    a, b, c; // sorted atom ids
-            float3 q;       // point of dE (or of the vdW sphere)
-            float  value;
-        };
-
-        struct SdfSmem
-        {
-            unsigned long long key[ kSdfList ];   // (delta bits << 32) | atom
-            float4             nb[ kSdfStaged ];   // neighbourhood of the atom being examined: (c_k, R_k)
-            uint16_t           near[ kNbrBuf ];    // its slots whose SAS sphere comes within the current best of x
-            uint8_t            vis[ kNbrBuf ];     // status of its circles
-        };
-
-        // neighbour slot s of atom i as (c_k, R_k): staged slots from shared memory
-        __device__ __forceinline__ float4 sdf_nb( const Build & b, const SdfSmem & sm, size_t row, uint32_t s )
-        {
-            if ( s < (uint32_t)kSdfStaged )
-                return sm.nb[ s ];
-            const float4 c = b.atoms[ b.nbr[ row + s ] ];
-            return make_float4( c.x, c.y, c.z, c.w + b.rp );
-        }
-
-        __device__ __forceinline__ void warp_min_hit( float & best, int & owner )
-        {
-            // smallest candidate distance, lowest lane on ties
-            for ( int o = 16; o > 0; o >>= 1 )
-            {
-                const float ob = __shfl_xor_sync( 0xffffffffu, best, o );
-                const int   oo = __shfl_xor_sync( 0xffffffffu, owner, o );
-                if ( ob < best || ( ob == best && oo < owner ) )
-                {
-                    best  = ob;
-                    owner = oo;
-                }
-            }
-        }
-
-        // Float32 error bound of |q - c_k|^2 - R_k^2 for a point q computed in absolute float32
-        // coordinates: a few ulps of the coordinates (at most qQ / 4, the query's largest coordinate
-        // plus its reach) on every coordinate, times 2 |q - c_k| (taken as R_k: the bound matters only
-        // where |q - c_k| is close to R_k), plus the rounding of the squares. Inside it the test is
-        // taken again in double precision.
-        __device__ __forceinline__ float hidden_band( float qQ, float d2, float Rk )
-        {
-            return 3.8147e-6f * ( d2 + Rk * ( Rk + qQ ) + 1.f );
-        }
-
-        // point q (double) strictly inside the SAS sphere of atom k, in double precision
-        __device__ __noinline__ bool point_inside_d( const Build & b, d3 q, uint32_t k )
-        {
-            const float4 ck = b.atoms[ k ];
-            const double Rk = (double)ck.w + (double)b.rp;
-            const double dx = q.x - (double)ck.x, dy = q.y - (double)ck.y, dz = q.z - (double)ck.z;
-            return dx * dx + dy * dy + dz * dz < Rk * Rk;
-        }
-
-        // The radial projection of x on the SAS sphere of i, in double precision, strictly inside the
-        // SAS sphere of one of this lane's near neighbours (lanes take every 32nd)
-        __device__ __noinline__ bool sphere_point_hidden_d( const Build & b, const SdfSmem & sm, size_t row, uint32_t nn,
-                                                            uint32_t i, float3 x, uint32_t lane )
-        {
-            const float4 ci = b.atoms[ i ];
-            const d3     wd = D3( (double)x.x - (double)ci.x, (double)x.y - (double)ci.y, (double)x.z - (double)ci.z );
-            const double Rd = (double)ci.w + (double)b.rp;
-            const double sc = Rd / sqrt( wd.x * wd.x + wd.y * wd.y + wd.z * wd.z );
-            const d3     qd = D3( (double)ci.x + wd.x * sc, (double)ci.y + wd.y * sc, (double)ci.z + wd.z * sc );
-            bool         hd = false;
-            for ( uint32_t e = lane; e < nn; e += 32 )
-                hd = hd || point_inside_d( b, qd, b.nbr[ row + sm.near[ e ] ] );
-            return hd;
-        }
-
-        // The nearest point of circle (i, neighbour slot s) to x, in double precision, strictly inside
-        // the SAS sphere of a near neighbour of i other than that of slot s
-        __device__ __noinline__ bool circle_point_hidden_d( const Build & b, const SdfSmem & sm, size_t row, uint32_t nn,
-                                                            uint32_t i, uint32_t s, float3 x )
-        {
-            const float4 ai = b.atoms[ i ], aj = b.atoms[ b.nbr[ row + s ] ];
-            const double Ri = (double)ai.w + (double)b.rp, Rj = (double)aj.w + (double)b.rp;
-            const d3     d  = D3( (double)aj.x - (double)ai.x, (double)aj.y - (double)ai.y, (double)aj.z - (double)ai.z );
-            const double dd = d.x * d.x + d.y * d.y + d.z * d.z;
-            const double tt = ( Ri * Ri - Rj * Rj + dd ) / ( 2.0 * dd );
-            const double r2 = Ri * Ri - tt * tt * dd;
-            if ( !( r2 > 0.0 ) )
-                return false;
-            const double r   = sqrt( r2 );
-            const double inv = 1.0 / sqrt( dd );
-            const d3     n   = D3( d.x * inv, d.y * inv, d.z * inv );
-            const d3     c   = D3( (double)ai.x + d.x * tt, (double)ai.y + d.y * tt, (double)ai.z + d.z * tt );
-            const d3     w   = D3( (double)x.x - c.x, (double)x.y - c.y, (double)x.z - c.z );
-            const double h   = w.x * n.x + w.y * n.y + w.z * n.z;
-            const d3     v   = D3( w.x - h * n.x, w.y - h * n.y, w.z - h * n.z );
-            const double rho = sqrt( v.x * v.x + v.y * v.y + v.z * v.z );
-            if ( !( rho > 0.0 ) )
-                return false;
-            const d3 q = D3( c.x + v.x * ( r / rho ), c.y + v.y * ( r / rho ), c.z + v.z * ( r / rho ) );
-            for ( uint32_t e = 0; e < nn; e++ )
-            {
-                const uint32_t k = sm.near[ e ];
-                if ( k != s && point_inside_d( b, q, b.nbr[ row + k ] ) )
-                    return true;
-            }
-            return false;
-        }
-
-        // one query, the whole warp; the hit is valid in every lane. A point of dE within the float32
-        // error of another SAS sphere is decided in double precision with kExact; without it the
-        // query is only marked (exact set, in every lane), for a second pass that runs it with kExact.
-        template<bool kExact>
-        __device__ SdfHit sdf_query( const Build & b, float3 x, SdfSmem & sm, float band, uint32_t & overflow, bool & exact )
-        {
-            const uint32_t lane      = lane_id();
-            bool           exactLane = false;
-            exact                    = false;
-            // 4 x (largest coordinate of any point of dE this query examines)
-            const float qQ = 4.f * ( fmaxf( fabsf( x.x ), fmaxf( fabsf( x.y ), fabsf( x.z ) ) ) + 12.f );
-            const float    T    = b.rp + band;
-            const FineGrid g    = b.fine[ 0 ];
-            Rows           rows;
-            stencil_rows( g, b.cellStart, fine_cell( g, x.x, x.y, x.z ), rows );
-            // atoms within reach; minima of |x - c| - R (SAS) and |x - c| - r (vdW)
-            uint32_t nl = 0;
-            float    smin = 3.4e38f, vmin = 3.4e38f;
-            int      vatom = 0x7fffffff;
-            for ( uint32_t base = 0; base < rows.total; base += 32 )
-            {
-                const uint32_t f    = base + lane;
-                bool           keep = false;
-                uint32_t       i    = 0;
-                float          dl   = 0.f;
-                if ( f < rows.total )
-                {
-                    const uint32_t idx = row_item( rows, f );
-                    i                  = b.cellItems[ idx ];
-                    const float4 c     = b.cellPos[ idx ];
-                    const float  ra    = fabsf( c.w );
-                    const float  L     = sqrtf( ( x.x - c.x ) * ( x.x - c.x ) + ( x.y - c.y ) * ( x.y - c.y ) + ( x.z - c.z ) * ( x.z - c.z ) );
-                    const float  R     = ra + b.rp;
-                    if ( L <= R + T )
-                    {
-                        smin = fminf( smin, L - R );
-                        const float v = L - ra;
-                        if ( v < vmin || ( v == vmin && (int)i < vatom ) )
-                        {
-                            vmin  = v;
-                            vatom = (int)i;
-                        }
-                        dl = fabsf( L - R );
-                        // fully buried atoms carry no point of dE: only the bounds above use them
-                        keep = !signbit( c.w );
-                    }
-                }
-                const uint32_t mk = __ballot_sync( 0xffffffffu, keep );
-                const uint32_t at = nl + __popc( mk & lanemask_lt() );
-                if ( keep && at < (uint32_t)kSdfList )
-                    sm.key[ at ] = ( (unsigned long long)__float_as_uint( dl ) << 32 ) | i;
-                nl += __popc( mk );
-            }
-            if ( nl > (uint32_t)kSdfList )
-            {
-                overflow = 1;
-                nl       = kSdfList;
-            }
-            for ( int o = 16; o > 0; o >>= 1 )
-            {
-                smin          = fminf( smin, __shfl_xor_sync( 0xffffffffu, smin, o ) );
-                const float v = __shfl_xor_sync( 0xffffffffu, vmin, o );
-                const int   a = __shfl_xor_sync( 0xffffffffu, vatom, o );
-                if ( v < vmin || ( v == vmin && a < vatom ) )
-                {
-                    vmin  = v;
-                    vatom = a;
-                }
-            }
-            SdfHit hit;
-            hit.a = hit.b = hit.c = -1;
-            hit.q                 = x;
-            if ( !( smin < 0.f ) )
-            {
-                // outside the SAS (or nothing within reach)
-                if ( vatom != 0x7fffffff && vmin <= band )
-                {
-                    hit.kind  = kSdfAtom;
-                    hit.a     = vatom;
-                    hit.value = vmin;
-                }
-                else
-                {
-                    hit.kind  = kSdfClampOutside;
-                    hit.value = band;
-                }
-                return hit;
-            }
-            __syncwarp();
-            float best  = T;
-            hit.kind    = kSdfClampInside;
-            // x lies in a SAS sphere with R - |x - c| = -smin: every point of dE is at least that far
-            const float floorD = -smin;
-            if ( !( floorD < T ) )
-            {
-                hit.value = b.rp - T;
-                return hit;
-            }
-            // probes (vertices of dE, never hidden) first: an early upper bound for the search
-            {
-                float  cand = 3.4e38f;
-                int    pa = -1, pb = -1, pc = -1;
-                float3 pq = x;
-                // lane per atom: its probe chunk
-                for ( uint32_t e0 = lane; e0 < nl; e0 += 32 )
-                {
-                    const uint32_t i     = (uint32_t)sm.key[ e0 ];
-                    const uint32_t chunk = b.chunkStart[ i ], len = b.chunkLen[ i ];
-                    for ( uint32_t e = 0; e < len; e++ )
-                    {
-                        const int4 cid = b.stageCid[ chunk + e ];
-                        if ( cid.w == 0 )
-                            continue;
-                        const float4 p    = b.stagePos[ chunk + e ];
-                        const float  dist = sqrtf( ( x.x - p.x ) * ( x.x - p.x ) + ( x.y - p.y ) * ( x.y - p.y ) + ( x.z - p.z ) * ( x.z - p.z ) );
-                        if ( dist < cand )
-                        {
-                            const int4 ids = b.stageIds[ chunk + e ];
-                            cand           = dist;
-                            pa             = ids.x;
-                            pb             = ids.y;
-                            pc             = ids.z;
-                            pq             = make_float3( p.x, p.y, p.z );
-                        }
-                    }
-                }
-                float wbest = cand;
-                int   owner = (int)lane;
-                warp_min_hit( wbest, owner );
-                if ( wbest < best )
-                {
-                    best     = wbest;
-                    hit.kind = kSdfProbe;
-                    hit.a    = __shfl_sync( 0xffffffffu, pa, owner );
-                    hit.b    = __shfl_sync( 0xffffffffu, pb, owner );
-                    hit.c    = __shfl_sync( 0xffffffffu, pc, owner );
-                    hit.q.x  = __shfl_sync( 0xffffffffu, pq.x, owner );
-                    hit.q.y  = __shfl_sync( 0xffffffffu, pq.y, owner );
-                    hit.q.z  = __shfl_sync( 0xffffffffu, pq.z, owner );
-                }
-            }
-            // atoms in ascending |x - c| - R order (the lower bound of all their candidates),
-            // each picked by a warp minimum over the ones left, until the bound reaches best
-            for ( uint32_t t = 0; t < nl; t++ )
-            {
-                unsigned long long key = ~0ull;
-                uint32_t           at  = 0;
-                for ( uint32_t e = lane; e < nl; e += 32 )
-                    if ( sm.key[ e ] < key )
-                    {
-                        key = sm.key[ e ];
-                        at  = e;
-                    }
-                for ( int o = 16; o > 0; o >>= 1 )
-                {
-                    const unsigned long long ok = __shfl_xor_sync( 0xffffffffu, key, o );
-                    const uint32_t           oa = __shfl_xor_sync( 0xffffffffu, at, o );
-                    if ( ok < key )
-                    {
-                        key = ok;
-                        at  = oa;
-                    }
-                }
-                const float dl = __uint_as_float( (uint32_t)( key >> 32 ) );
-                if ( !( dl < best ) || !( floorD < best ) )
-                    break; // every candidate of this and the remaining atoms is at least dl away
-                __syncwarp();
-                if ( lane == 0 )
-                    sm.key[ at ] = ~0ull; // taken
-                const uint32_t i   = (uint32_t)key;
-                const float4   ci  = b.atoms[ i ];
-                const float    Ri  = ci.w + b.rp;
-                const uint32_t ni  = b.nbrCount[ i ];
-                const size_t   row = (size_t)i * b.cap;
-                // stage N(i); a point q with |x - q| < best can only lie inside the SAS
-                // sphere of a neighbour k with |x - c_k| - R_k < best: those are the "near" ones
-                uint32_t nn = 0;
-                for ( uint32_t s0 = 0; s0 < ni; s0 += 32 )
-                {
-                    const uint32_t s    = s0 + lane;
-                    bool           near = false;
-                    if ( s < ni )
-                    {
-                        sm.vis[ s ]     = b.status[ row + s ];
-                        const float4 ck = b.atoms[ b.nbr[ row + s ] ];
-                        const float  Rk = ck.w + b.rp;
-                        if ( s < (uint32_t)kSdfStaged )
-                            sm.nb[ s ] = make_float4( ck.x, ck.y, ck.z, Rk );
-                        const float Lk  = sqrtf( ( x.x - ck.x ) * ( x.x - ck.x ) + ( x.y - ck.y ) * ( x.y - ck.y ) + ( x.z - ck.z ) * ( x.z - ck.z ) );
-                        near            = Lk - Rk < best;
-                    }
-                    const uint32_t mk = __ballot_sync( 0xffffffffu, near );
-                    if ( near )
-                        sm.near[ nn + __popc( mk & lanemask_lt() ) ] = (uint16_t)s;
-                    nn += __popc( mk );
-                }
-                __syncwarp();
-                // candidates of this atom, one per lane at most, reduced at the end
-                float  cand = 3.4e38f;
-                int    ck = 0, cb = -1, cc = -1;
-                float3 cq = x;
-                // radial projection on sphere i
-                {
-                    const float3 w = make_float3( x.x - ci.x, x.y - ci.y, x.z - ci.z );
-                    const float  L = sqrtf( w.x * w.x + w.y * w.y + w.z * w.z );
-                    if ( L > 0.f )
-                    {
-                        const float3 q = make_float3( ci.x + w.x * ( Ri / L ), ci.y + w.y * ( Ri / L ), ci.z + w.z * ( Ri / L ) );
-                        bool         hidden = false, unsure = false;
-                        for ( uint32_t e = lane; e < nn; e += 32 )
-                        {
-                            const float4 nk = sdf_nb( b, sm, row, sm.near[ e ] );
-                            const float  dx = q.x - nk.x, dy = q.y - nk.y, dz = q.z - nk.z;
-                            const float  d2 = dx * dx + dy * dy + dz * dz;
-                            const float  m  = d2 - nk.w * nk.w;
-                            const float  eb = hidden_band( qQ, d2, nk.w );
-                            hidden          = hidden || m < -eb;
-                            unsure          = unsure || !( fabsf( m ) > eb );
-                        }
-                        bool hid = __any_sync( 0xffffffffu, hidden );
-                        if ( !hid && __any_sync( 0xffffffffu, unsure ) )
-                        {
-                            // a neighbour's sphere passes within the float32 error of the point:
-                            // the point and the test in double precision
-                            if ( kExact )
-                                hid = __any_sync( 0xffffffffu, sphere_point_hidden_d( b, sm, row, nn, i, x, lane ) );
-                            else
-                                exactLane = true;
-                        }
-                        if ( !hid && lane == 0 )
-                        {
-                            cand = dl;
-                            ck   = kSdfSphere;
-                            cq   = q;
-                        }
-                    }
-                }
-                // nearest points of the visible circles of i
-                for ( uint32_t s0 = 0; s0 < ni; s0 += 32 )
-                {
-                    const uint32_t s = s0 + lane;
-                    if ( s >= ni || sm.vis[ s ] == 0 )
-                        continue;
-                    const float4 nj = sdf_nb( b, sm, row, s );
-                    {
-                        // every point of circle (i, j) is on sphere j too: |x - c_j| - R_j bounds it
-                        const float Lj = sqrtf( ( x.x - nj.x ) * ( x.x - nj.x ) + ( x.y - nj.y ) * ( x.y - nj.y ) + ( x.z - nj.z ) * ( x.z - nj.z ) );
-                        if ( !( fabsf( Lj - nj.w ) < best ) )
-                            continue;
-                    }
-                    const float3 d  = make_float3( nj.x - ci.x, nj.y - ci.y, nj.z - ci.z );
-                    const float  dd = d.x * d.x + d.y * d.y + d.z * d.z;
-                    const float  tt = ( Ri * Ri - nj.w * nj.w + dd ) / ( 2.f * dd );
-                    const float  r2 = Ri * Ri - tt * tt * dd;
-                    if ( !( r2 > 0.f ) )
-                        continue;
-                    const float  r   = sqrtf( r2 );
-                    const float  inv = rsqrtf( dd );
-                    const float3 n   = make_float3( d.x * inv, d.y * inv, d.z * inv );
-                    const float3 c   = make_float3( ci.x + d.x * tt, ci.y + d.y * tt, ci.z + d.z * tt );
-                    const float3 w   = make_float3( x.x - c.x, x.y - c.y, x.z - c.z );
-                    const float  h   = w.x * n.x + w.y * n.y + w.z * n.z;
-                    const float3 v   = make_float3( w.x - h * n.x, w.y - h * n.y, w.z - h * n.z );
-                    const float  rho = sqrtf( v.x * v.x + v.y * v.y + v.z * v.z );
-                    float        dist;
-                    float3       q = c;
-                    if ( rho > 1e-6f )
-                    {
-                        q    = make_float3( c.x + v.x * ( r / rho ), c.y + v.y * ( r / rho ), c.z + v.z * ( r / rho ) );
-                        dist = sqrtf( h * h + ( rho - r ) * ( rho - r ) );
-                        if ( !( dist < cand ) || !( dist < best ) )
-                            continue;
-                        bool hidden = false, unsure = false;
-                        for ( uint32_t e = 0; e < nn && !hidden; e++ )
-                        {
-                            const uint32_t k = sm.near[ e ];
-                            if ( k == s )
-                                continue;
-                            const float4 nk = sdf_nb( b, sm, row, k );
-                            const float  dx = q.x - nk.x, dy = q.y - nk.y, dz = q.z - nk.z;
-                            const float  d2 = dx * dx + dy * dy + dz * dz;
-                            const float  m  = d2 - nk.w * nk.w;
-                            const float  eb = hidden_band( qQ, d2, nk.w );
-                            hidden          = m < -eb;
-                            unsure          = unsure || !( fabsf( m ) > eb );
-                        }
-                        if ( !hidden && unsure )
-                        {
-                            if ( kExact )
-                                hidden = circle_point_hidden_d( b, sm, row, nn, i, s, x );
-                            else
-                                exactLane = true;
-                        }
-                        if ( hidden )
-                            continue;
-                    }
-                    else
-                    {
-                        // x on the axis: every point of the circle is as near; a visible
-                        // circle has an accessible arc
-                        dist = sqrtf( h * h + r2 );
-                        if ( !( dist < cand ) || !( dist < best ) )
-                            continue;
-                    }
-                    cand = dist;
-                    ck   = kSdfCircle;
-                    cb   = (int)b.nbr[ row + s ];
-                    cq   = q;
-                }
-                float wbest = cand;
-                int   owner = (int)lane;
-                warp_min_hit( wbest, owner );
-                if ( wbest < best )
-                {
-                    best     = wbest;
-                    hit.kind = __shfl_sync( 0xffffffffu, ck, owner );
-                    hit.a    = (int)i;
-                    hit.b    = __shfl_sync( 0xffffffffu, cb, owner );
-                    hit.c    = __shfl_sync( 0xffffffffu, cc, owner );
-                    hit.q.x  = __shfl_sync( 0xffffffffu, cq.x, owner );
-                    hit.q.y  = __shfl_sync( 0xffffffffu, cq.y, owner );
-                    hit.q.z  = __shfl_sync( 0xffffffffu, cq.z, owner );
-                }
-                __syncwarp();
-            }
-            hit.value = b.rp - best;
-            exact     = __any_sync( 0xffffffffu, exactLane );
-            return hit;
-        }
-
-        __device__ __forceinline__ void add_grad( float * g, uint32_t atom, float gx, float gy, float gz, float gr )
-        {
-            atomicAdd( g + 4 * atom + 0, gx );
-            atomicAdd( g + 4 * atom + 1, gy );
-            atomicAdd( g + 4 * atom + 2, gz );
-            atomicAdd( g + 4 * atom + 3, gr );
-        }
-
-        // d sdf / d (c, r) of the active primitive, scaled by gs, into g (sorted order)
-        __device__ __noinline__ void sdf_gradient( const Build & b, const SdfHit & h, float3 x, float gs, float * g )
-        {
-            if ( h.kind == kSdfAtom || h.kind == kSdfSphere )
-            {
-                // sdf = |x - c_a| - r_a (outside the SAS, or x inside sphere a); the
-                // opposite sign when x lies outside sphere a but inside another
-                const float4 c = b.atoms[ h.a ];
-                const float3 w = make_float3( x.x - c.x, x.y - c.y, x.z - c.z );
-                const float  L = sqrtf( w.x * w.x + w.y * w.y + w.z * w.z );
-                if ( !( L > 0.f ) )
-                    return;
-                float sgn = -1.f;
-                if ( h.kind == kSdfSphere && L > c.w + b.rp )
-                    sgn = 1.f;
-                add_grad( g, (uint32_t)h.a, gs * sgn * w.x / L, gs * sgn * w.y / L, gs * sgn * w.z / L, gs * sgn );
-                return;
-            }
-            if ( h.kind != kSdfCircle && h.kind != kSdfProbe )
-                return;
-            // The multipliers of the constraints |p - c_k|^2 = R_k^2 that hold the point p: a 2x2
-            // (circle) or 3x3 (probe) system that is nearly singular when the constraint normals
-            // are nearly parallel (two circle centres nearly aligned with p, a probe near the plane
-            // of its three centres), where float32 would show in the gradient. Solved in double
-            // precision from the float32 values (their differences are exact in double); one lane
-            // per query, so the FP64 pipe's rate does not matter.
-            const float3 pf = h.q;
-            const d3     p  = D3( (double)pf.x, (double)pf.y, (double)pf.z );
-            const d3     dv = D3( (double)x.x - p.x, (double)x.y - p.y, (double)x.z - p.z );
-            const double D  = sqrt( dv.x * dv.x + dv.y * dv.y + dv.z * dv.z );
-            if ( !( D > 0.0 ) )
-                return;
-            const d3  u = D3( dv.x / D, dv.y / D, dv.z / D );
-            const int m = h.kind == kSdfCircle ? 2 : 3;
-            const int ids[ 3 ] = { h.a, h.b, h.c };
-            d3        a[ 3 ];
-            double    R[ 3 ];
-            for ( int k = 0; k < m; k++ )
-            {
-                const float4 c = b.atoms[ ids[ k ] ];
-                a[ k ]         = D3( 2.0 * ( p.x - (double)c.x ), 2.0 * ( p.y - (double)c.y ), 2.0 * ( p.z - (double)c.z ) );
-                R[ k ]         = (double)c.w + (double)b.rp;
-            }
-            // multipliers w: sum_k w_k a_k = u (least squares for the circle, exact for the probe)
-            double w[ 3 ] = { 0.0, 0.0, 0.0 };
-            if ( m == 2 )
-            {
-                const double g00 = a[ 0 ].x * a[ 0 ].x + a[ 0 ].y * a[ 0 ].y + a[ 0 ].z * a[ 0 ].z;
-                const double g01 = a[ 0 ].x * a[ 1 ].x + a[ 0 ].y * a[ 1 ].y + a[ 0 ].z * a[ 1 ].z;
-                const double g11 = a[ 1 ].x * a[ 1 ].x + a[ 1 ].y * a[ 1 ].y + a[ 1 ].z * a[ 1 ].z;
-                const double r0  = a[ 0 ].x * u.x + a[ 0 ].y * u.y + a[ 0 ].z * u.z;
-                const double r1  = a[ 1 ].x * u.x + a[ 1 ].y * u.y + a[ 1 ].z * u.z;
-                const double det = g00 * g11 - g01 * g01;
-                if ( !( fabs( det ) > 0.0 ) )
-                    return;
-                w[ 0 ] = ( r0 * g11 - r1 * g01 ) / det;
-                w[ 1 ] = ( r1 * g00 - r0 * g01 ) / det;
-            }
-            else
-            {
-                // columns a_0, a_1, a_2: Cramer's rule
-                const d3     c12 = dcross( a[ 1 ], a[ 2 ] );
-                const double det = ddot( a[ 0 ], c12 );
-                if ( !( fabs( det ) > 0.0 ) )
-                    return;
-                w[ 0 ] = ddot( u, c12 ) / det;                    // det[u, a1, a2]
-                w[ 1 ] = ddot( a[ 0 ], dcross( u, a[ 2 ] ) ) / det; // det[a0, u, a2]
-                w[ 2 ] = ddot( dcross( a[ 0 ], a[ 1 ] ), u ) / det; // det[a0, a1, u]
-            }
-            // sdf = rp - D: d sdf / d c_k = w_k a_k, d sdf / d r_k = 2 w_k R_k
-            for ( int k = 0; k < m; k++ )
-                add_grad( g, (uint32_t)ids[ k ], (float)( gs * w[ k ] * a[ k ].x ), (float)( gs * w[ k ] * a[ k ].y ),
-                          (float)( gs * w[ k ] * a[ k ].z ), (float)( gs * 2.0 * w[ k ] * R[ k ] ) );
-        }
-
-        // grid cell of each query (sort key) and its index
-        __global__ void k_sdf_keys( Build b, const float * queries, uint32_t m, uint32_t * keys, uint32_t * order )
-        {
-            const FineGrid g = b.fine[ 0 ];
-            for ( uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x )
-            {
-                keys[ q ]  = fine_key( g, fine_cell( g, queries[ 3 * (size_t)q ], queries[ 3 * (size_t)q + 1 ], queries[ 3 * (size_t)q + 2 ] ) );
-                order[ q ] = q;
-            }
-        }
-
-        // First pass over the queries (in grid-cell order: neighbouring warps read the same atoms);
-        // a query that needs a double-precision decision is listed for k_sdf_exact instead
-        template<bool kBackward>
-        __global__ void __launch_bounds__( 32 * kSdfWarps, 8 ) k_sdf( Build b, const float * queries, uint32_t m, float band,
-                                                                   float * sdf, const float * gradSdf, float * gradSorted,
-                                                                   int * kind, const uint32_t * order, uint32_t * exactList,
-                                                                   uint32_t * exactCount )
-        {
-            __shared__ SdfSmem smem[ kSdfWarps ];
-            const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
-            uint32_t           overflow = 0;
-            for ( uint32_t qs = blockIdx.x * kSdfWarps + warp; qs < m; qs += gridDim.x * kSdfWarps )
-            {
-                const uint32_t qi = order[ qs ];
-                const float3 x = make_float3( queries[ 3 * (size_t)qi ], queries[ 3 * (size_t)qi + 1 ], queries[ 3 * (size_t)qi + 2 ] );
-                bool         exact;
-                const SdfHit h = sdf_query<false>( b, x, smem[ warp ], band, overflow, exact );
-                if ( lane == 0 )
-                {
-                    if ( exact )
-                        exactList[ atomicAdd( exactCount, 1u ) ] = qi;
-                    else if ( kBackward )
-                        sdf_gradient( b, h, x, gradSdf[ qi ], gradSorted );
-                    else
-                    {
-                        sdf[ qi ] = h.value;
-                        if ( kind )
-                            kind[ qi ] = h.kind;
-                    }
-                }
-            }
-            if ( lane == 0 && overflow )
-                atomicOr( &b.counts->overflow, (uint32_t)kOverflowSdfList );
-        }
-
-        // Second pass: the listed queries, with every decision within the float32 band taken in
-        // double precision (few queries: a point of dE next to another SAS sphere's surface)
-        template<bool kBackward>
-        __global__ void __launch_bounds__( 32 * kSdfWarps ) k_sdf_exact( Build b, const float * queries, float band, float * sdf,
-                                                                      const float * gradSdf, float * gradSorted, int * kind,
-                                                                      const uint32_t * exactList, const uint32_t * exactCount )
-        {
-            __shared__ SdfSmem smem[ kSdfWarps ];
-            const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
-            const uint32_t     count = *exactCount;
-            uint32_t           overflow = 0;
-            for ( uint32_t e = blockIdx.x * kSdfWarps + warp; e < count; e += gridDim.x * kSdfWarps )
-            {
-                const uint32_t qi = exactList[ e ];
-                const float3 x = make_float3( queries[ 3 * (size_t)qi ], queries[ 3 * (size_t)qi + 1 ], queries[ 3 * (size_t)qi + 2 ] );
-                bool         exact;
-                const SdfHit h = sdf_query<true>( b, x, smem[ warp ], band, overflow, exact );
-                if ( lane == 0 )
-                {
-                    if ( kBackward )
-                        sdf_gradient( b, h, x, gradSdf[ qi ], gradSorted );
-                    else
-                    {
-                        sdf[ qi ] = h.value;
-                        if ( kind )
-                            kind[ qi ] = h.kind;
-                    }
-                }
-            }
-            if ( lane == 0 && overflow )
-                atomicOr( &b.counts->overflow, (uint32_t)kOverflowSdfList );
-        }
-
-        __global__ void k_sdf_unsort( Build b, const float * gradSorted, float * gradInput )
-        {
-            for ( uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < b.n; s += gridDim.x * blockDim.x )
-            {
-                const uint32_t i = b.perm[ s ];
-                for ( int k = 0; k < 4; k++ )
-                    gradInput[ 4 * (size_t)i + k ] = gradSorted[ 4 * (size_t)s + k ];
-            }
-        }
-
-        // ---- headless image: sphere tracing of the signed distance ------------------
-        // Every pixel's ray x(t) = eye + t d advances by a step that never crosses the SES:
-        // inside the SAS (kinds 3-5) the value rp - dist(x, E) bounds the distance to the SES
-        // (every SES point lies at rp from E); outside (kinds 1, 2) value - rp bounds the distance
-        // to the SAS, which holds the SES. A ray stops when an inside value falls below eps (a hit
-        // at t), when it reaches a point deeper than the band (kind 0, taken as a hit), or when t
-        // passes tFar; it advances by at least eps / 4. The ray setup, the march (points eye + t d,
-        // steps, t) and the normals are in float32 with every operation rounded on its own, in the
-        // order the host tracer writes them, so that the image does not depend on contraction
-        // choices. The normal of a hit is the normalised central difference of the signed distance
-        // (step normalStep) at the hit point.
-        __global__ void __launch_bounds__( 32 * kSdfWarps ) k_trace( Build b, TraceParams p, float band, float * depth,
-                                                                       float * normals )
-        {
-            __shared__ SdfSmem smem[ kSdfWarps ];
-            const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
-            uint32_t           overflow = 0;
-            const uint32_t     pixels   = p.width * p.height;
-            const float3       f        = make_float3( (float)p.forward[ 0 ], (float)p.forward[ 1 ], (float)p.forward[ 2 ] );
-            const float3       r        = make_float3( (float)p.right[ 0 ], (float)p.right[ 1 ], (float)p.right[ 2 ] );
-            const float3       u        = make_float3( (float)p.up[ 0 ], (float)p.up[ 1 ], (float)p.up[ 2 ] );
-            const float3       ef       = make_float3( (float)p.eye[ 0 ], (float)p.eye[ 1 ], (float)p.eye[ 2 ] );
-            const float        th       = (float)p.tanHalfFov, W = (float)p.width, H = (float)p.height;
-            const float        eps      = (float)p.eps, tFar = (float)p.tFar, hn = (float)p.normalStep;
-            const float        minStep  = __fmul_rn( 0.25f, eps );
-            for ( uint32_t px = blockIdx.x * kSdfWarps + warp; px < pixels; px += gridDim.x * kSdfWarps )
-            {
-                const uint32_t iy = px / p.width, ix = px - iy * p.width;
-                // pinhole ray through the pixel centre, row-major from the top left
-                const float xs  = __fdiv_rn( __fmul_rn( __fmul_rn( __fsub_rn( __fdiv_rn( __fmul_rn( 2.f, __fadd_rn( (float)ix, 0.5f ) ), W ), 1.f ),
-                                                                  th ),
-                                                        W ),
-                                             H );
-                const float ys  = __fmul_rn( __fsub_rn( 1.f, __fdiv_rn( __fmul_rn( 2.f, __fadd_rn( (float)iy, 0.5f ) ), H ) ), th );
-                const float dx  = __fadd_rn( __fadd_rn( f.x, __fmul_rn( r.x, xs ) ), __fmul_rn( u.x, ys ) );
-                const float dy  = __fadd_rn( __fadd_rn( f.y, __fmul_rn( r.y, xs ) ), __fmul_rn( u.y, ys ) );
-                const float dz  = __fadd_rn( __fadd_rn( f.z, __fmul_rn( r.z, xs ) ), __fmul_rn( u.z, ys ) );
-                const float len = __fsqrt_rn( __fadd_rn( __fadd_rn( __fmul_rn( dx, dx ), __fmul_rn( dy, dy ) ), __fmul_rn( dz, dz ) ) );
-                const float3 df = make_float3( __fdiv_rn( dx, len ), __fdiv_rn( dy, len ), __fdiv_rn( dz, len ) );
-                float        t   = (float)p.tNear;
-                float        hit = __int_as_float( 0x7f800000 ); // +inf: background
-                // One query call site for the march and the six evaluations of the normal (the
-                // query is inlined once). Evaluation k of the normal moves the hit point by +hn
-                // (k even) or -hn (k odd) along axis k / 2.
-                float3   xh = make_float3( 0.f, 0.f, 0.f ), g = make_float3( 0.f, 0.f, 0.f );
-                float    vp = 0.f;
-                uint32_t step = 0;
-                int      k    = -1; // -1: marching
-                while ( true )
-                {
-                    float3 q;
-                    if ( k < 0 )
-                    {
-                        if ( !( step < p.maxSteps && t <= tFar ) )
-                            break;
-                        q = make_float3( __fadd_rn( ef.x, __fmul_rn( t, df.x ) ), __fadd_rn( ef.y, __fmul_rn( t, df.y ) ),
-                                         __fadd_rn( ef.z, __fmul_rn( t, df.z ) ) );
-                    }
-                    else
-                    {
-                        if ( k == 6 )
-                            break;
-                        const float e = ( k & 1 ) ? -hn : hn;
-                        q             = xh;
-                        if ( k < 2 )
-                            q.x = __fadd_rn( xh.x, e );
-                        else if ( k < 4 )
-                            q.y = __fadd_rn( xh.y, e );
-                        else
-                            q.z = __fadd_rn( xh.z, e );
-                    }
-                    bool         ex;
-                    const SdfHit h = sdf_query<true>( b, q, smem[ warp ], band, overflow, ex );
-                    if ( k < 0 )
-                    {
-                        step++;
-                        const bool inside = h.kind == kSdfSphere || h.kind == kSdfCircle || h.kind == kSdfProbe;
-                        if ( ( inside && h.value < eps ) || h.kind == kSdfClampInside )
-                        {
-                            hit = t;
-                            if ( !normals )
-                                break;
-                            // the hit point as the march computed it
-                            xh = q;
-                            k  = 0;
-                            continue;
-                        }
-                        const float st = inside ? h.value : __fsub_rn( h.value, b.rp );
-                        t              = __fadd_rn( t, fmaxf( st, minStep ) );
-                        continue;
-                    }
-                    if ( ( k & 1 ) == 0 )
-                        vp = h.value;
-                    else
-                    {
-                        const float ga = __fdiv_rn( __fsub_rn( vp, h.value ), __fmul_rn( 2.f, hn ) );
-                        if ( k == 1 )
-                            g.x = ga;
-                        else if ( k == 3 )
-                            g.y = ga;
-                        else
-                            g.z = ga;
-                    }
-                    k++;
-                }
-                float3 nrm = make_float3( 0.f, 0.f, 0.f );
-                if ( normals && hit < 3.4e38f )
-                {
-                    const float gl  = __fsqrt_rn( __fadd_rn( __fadd_rn( __fmul_rn( g.x, g.x ), __fmul_rn( g.y, g.y ) ), __fmul_rn( g.z, g.z ) ) );
-                    const float inv = gl > 0.f ? gl : 1.f;
-                    nrm = make_float3( __fdiv_rn( g.x, inv ), __fdiv_rn( g.y, inv ), __fdiv_rn( g.z, inv ) );
-                }
-                if ( lane == 0 )
-                {
-                    depth[ px ] = hit;
-                    if ( normals )
-                    {
-                        normals[ 3 * (size_t)px ]     = nrm.x;
-                        normals[ 3 * (size_t)px + 1 ] = nrm.y;
-                        normals[ 3 * (size_t)px + 2 ] = nrm.z;
-                    }
-                }
-            }
-            if ( lane == 0 && overflow )
-                atomicOr( &b.counts->overflow, (uint32_t)kOverflowSdfList );
-        }
-    } // namespace
-
-    // keys and order of the queries, the list of queries for the exact pass and its counter, radix scratch
-    size_t sdf_scratch_bytes( uint32_t m ) { return 3 * ( ( (size_t)m * 4 + 255 ) & ~(size_t)255 ) + 256 + radix_scratch_bytes( m ); }
-
-    // the list of queries for the exact pass (m entries, then its counter)
-    static uint32_t * sdf_exact_list( void * scratch, uint32_t m )
-    {
-        return reinterpret_cast<uint32_t *>( static_cast<char *>( scratch ) + 2 * ( ( (size_t)m * 4 + 255 ) & ~(size_t)255 ) );
-    }
-
-    // queries sorted by grid cell into `order` (scratch: sdf_scratch_bytes)
-    static const uint32_t * sdf_order( const Build & b, const float * queries, uint32_t m, void * scratch, cudaStream_t s )
-    {
-        char *     p     = static_cast<char *>( scratch );
-        uint32_t * keys  = reinterpret_cast<uint32_t *>( p );
-        uint32_t * order = reinterpret_cast<uint32_t *>( p + ( ( (size_t)m * 4 + 255 ) & ~(size_t)255 ) );
-        void *     rad   = p + 3 * ( ( (size_t)m * 4 + 255 ) & ~(size_t)255 ) + 256;
-        k_sdf_keys<<<min( persistent_blocks( 256 ), blocks_for( m, 256 ) ), 256, 0, s>>>( b, queries, m, keys, order );
-        counted();
-        radix_sort( keys, order, m, 32, rad, s );
-        return order;
-    }
-
-    void launch_sdf( const Build & b, const float * queries, uint32_t m, float band, float * sdf, int * kind, void * scratch,
-                     cudaStream_t s )
-    {
-        if ( !m )
-            return;
-        const uint32_t * order  = sdf_order( b, queries, m, scratch, s );
-        uint32_t *       list   = sdf_exact_list( scratch, m );
-        uint32_t *       count  = list + ( ( (size_t)m * 4 + 255 ) & ~(size_t)255 ) / 4;
-        const uint32_t   blocks = min( persistent_blocks( 32 * kSdfWarps ) * 2, ( m + kSdfWarps - 1 ) / kSdfWarps );
-        cudaMemsetAsync( count, 0, sizeof( uint32_t ), s );
-        k_sdf<false><<<blocks, 32 * kSdfWarps, 0, s>>>( b, queries, m, band, sdf, nullptr, nullptr, kind, order, list, count );
-        k_sdf_exact<false><<<min( blocks, 152u * 4u ), 32 * kSdfWarps, 0, s>>>( b, queries, band, sdf, nullptr, nullptr, kind, list,
-                                                                              count );
-        counted( 2 );
-    }
-    void launch_trace( const Build & b, const TraceParams & p, float band, float * depth, float * normals, cudaStream_t s )
-    {
-        const uint32_t pixels = p.width * p.height;
-        if ( !pixels )
-            return;
-        const uint32_t blocks = min( persistent_blocks( 32 * kSdfWarps ) * 2, ( pixels + kSdfWarps - 1 ) / kSdfWarps );
-        k_trace<<<blocks, 32 * kSdfWarps, 0, s>>>( b, p, band, depth, normals );
-        counted();
-    }
-
-    void launch_sdf_backward( const Build & b, const float * queries, uint32_t m, float band, const float * gradSdf,
-                              float * gradSorted, float * gradInput, void * scratch, cudaStream_t s )
-    {
-        cudaMemsetAsync( gradSorted, 0, sizeof( float ) * 4 * (size_t)b.n, s );
-        if ( m )
-        {
-            const uint32_t * order  = sdf_order( b, queries, m, scratch, s );
-            uint32_t *       list   = sdf_exact_list( scratch, m );
-            uint32_t *       count  = list + ( ( (size_t)m * 4 + 255 ) & ~(size_t)255 ) / 4;
-            const uint32_t   blocks = min( persistent_blocks( 32 * kSdfWarps ) * 2, ( m + kSdfWarps - 1 ) / kSdfWarps );
-            cudaMemsetAsync( count, 0, sizeof( uint32_t ), s );
-            k_sdf<true><<<blocks, 32 * kSdfWarps, 0, s>>>( b, queries, m, band, nullptr, gradSdf, gradSorted, nullptr, order, list,
-                                                           count );
-            k_sdf_exact<true><<<min( blocks, 152u * 4u ), 32 * kSdfWarps, 0, s>>>( b, queries, band, nullptr, gradSdf, gradSorted,
-                                                                                 nullptr, list, count );
-            counted( 2 );
-        }
-        if ( b.n )
-        {
-            k_sdf_unsort<<<blocks_for( b.n, 256 ), 256, 0, s>>>( b, gradSorted, gradInput );
-            counted();
-        }
     }
 } // namespace sesgb

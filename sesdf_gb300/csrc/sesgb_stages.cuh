@@ -124,26 +124,30 @@ namespace sesgb
     void launch_gather( const Build & b, cudaStream_t s );
     // zeroes a[0, n] and c[0, n] (c may be null) with n = min(*nDevice, nHost), or nHost without nDevice
     void launch_zero2( uint32_t * a, uint32_t * c, uint32_t nHost, const uint32_t * nDevice, cudaStream_t s );
-    // kind 0: the sorted atoms (n); kind 1: the singular probes (count read from *nDevice); kind 2: the
-    // sorted atoms with the radius negated for atoms without accessible surface (SDF queries)
+    // kind 0: the sorted atoms (n); kind 1: the singular probes (count read from *nDevice)
     void launch_cells( const Build & b, int kind, uint32_t nHost, const uint32_t * nDevice, void * scanScratch,
                        cudaStream_t s );
     void launch_batch_finish( const Build & b, cudaStream_t s );
-    // signed distance to the SES at float3 query points (needs the atom grid of reach
-    // rmax + 2 rp + band built by launch_fine_params + launch_cells first)
-    size_t sdf_scratch_bytes( uint32_t m );
-    void   launch_sdf( const Build & b, const float * queries, uint32_t m, float band, float * sdf, int * kind, void * scratch,
-                       cudaStream_t s );
-    void   launch_sdf_backward( const Build & b, const float * queries, uint32_t m, float band, const float * gradSdf,
+    // signed distance to the SES at float3 query points (sesgb_sdf.cu)
+    struct SdfState
+    {
+        float rmax;    // largest vdW radius of the build
+        bool  general; // truncated neighbour lists, or atoms outside the grid's box: the general search alone
+    };
+    size_t sdf_scratch_bytes( const Build & b, const SdfState & st, uint32_t m );
+    void   launch_sdf( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,
+                       void * scratch, cudaStream_t s );
+    void   launch_sdf_backward( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, const float * gradSdf,
                                 float * gradSorted, float * gradInput, void * scratch, cudaStream_t s );
-    // headless image: every pixel's ray sphere-traced against the signed distance (same grid as the SDF)
+    // headless image: every pixel's ray sphere-traced against the signed distance (scratch: sdf_scratch_bytes with m = 0)
     struct TraceParams
     {
         double   eye[ 3 ], forward[ 3 ], right[ 3 ], up[ 3 ];
         double   tanHalfFov, tNear, tFar, eps, normalStep;
         uint32_t width, height, maxSteps;
     };
-    void launch_trace( const Build & b, const TraceParams & p, float band, float * depth, float * normals, cudaStream_t s );
+    void launch_trace( const Build & b, const SdfState & st, const TraceParams & p, float band, float * depth, float * normals,
+                       void * scratch, cudaStream_t s );
     // components of the probe-accessible space on a voxel grid (sesgb_cavities.cu)
     struct CavGrid
     {

@@ -1,0 +1,91 @@
+"""The tile search of the signed distance against the general search, and against itself in other tiles.
+
+A context whose box leaves an atom outside takes the general search for every query (the tile search needs
+every atom inside the grid), so that the same molecule, with one more atom far from everything, gives the
+general search's values: the tile search's have to be the same float32 numbers, and so do its gradients to the
+rounding of their float32 sums. Query counts around the numbers of lanes a query gets (1 to 32) and of queries
+a tile holds; probe radii from small to larger than the band; radii and coordinates far from a protein's; points
+that are not numbers, far away, at atom centres and on probes."""
+import numpy as np
+import pytest
+
+from cases import hand_cases
+from sesdf_gb300 import SesBuild, synth
+from sesdf_gb300.api import aabb
+
+pytestmark = pytest.mark.gpu
+FAR = np.array([[400.0, 0.0, 0.0, 1.5]], np.float32)
+
+
+def evaluate(g, q, gq=None):
+    import torch
+    dq = torch.from_numpy(np.ascontiguousarray(q, np.float32)).cuda()
+    out = torch.empty(len(q), dtype=torch.float32, device="cuda")
+    kind = torch.empty(len(q), dtype=torch.int32, device="cuda")
+    g.sdf(dq.data_ptr(), len(q), out.data_ptr(), kind.data_ptr())
+    grad = None
+    if gq is not None:
+        dg = torch.from_numpy(np.ascontiguousarray(gq, np.float32)).cuda()
+        ga = torch.empty((g.atoms.shape[0], 4), dtype=torch.float32, device="cuda")
+        g.sdf_backward(dq.data_ptr(), len(q), dg.data_ptr(), ga.data_ptr())
+        grad = ga.cpu().numpy()
+    torch.cuda.synchronize()
+    return out.cpu().numpy(), kind.cpu().numpy(), grad
+
+
+def molecules():
+    shrunk = synth.globule(400, 21)
+    shrunk[:, 3] *= 0.5
+    coarse = synth.globule(600, 22)
+    coarse *= np.float32(3.0)  # beads of 5 A
+    moved = synth.globule(700, 23)
+    moved[:, :3] += np.float32([150.0, -90.0, 60.0])
+    dense = synth.globule(900, 24)
+    dense[:, :3] *= np.float32(0.6)
+    out = {"globule": (synth.globule(1500, 20), 1.4), "small_radii": (shrunk, 1.4), "beads": (coarse, 1.4), "moved": (moved, 1.2),
+           "dense": (dense, 1.4), "coarse_probe": (synth.globule(800, 25), 2.4), "large_probe": (synth.globule(500, 26), 3.6)}
+    for name in ("single", "pair", "collinear", "octahedron", "stack"):
+        out[name] = (hand_cases()[name], 1.4)
+    return out
+
+
+@pytest.mark.parametrize("name", sorted(molecules()))
+def test_tile_search_gives_the_general_search(name):
+    atoms, rp = molecules()[name]
+    atoms = np.concatenate([atoms, FAR + np.float32([*atoms[:, :3].mean(0), 0.0])])
+    plain = 3000
+    q = np.concatenate([synth.queries(atoms[:-1], plain, 31), atoms[:40, :3], atoms[:40, :3] + np.float32(1e-3),
+                        (atoms[:40, :3] + atoms[1:41, :3][: len(atoms[:40])]) * np.float32(0.5) if len(atoms) > 41 else atoms[:0, :3],
+                        np.float32([[np.nan, 0, 0], [np.inf, 0, 0], [1e6, 1e6, -1e6], [0, 1e30, 0]])])
+    rng = np.random.default_rng(5)
+    with SesBuild(atoms, rp, "full", max_neighbor_per_atom=288) as tile, \
+            SesBuild(atoms, rp, "full", box=aabb(atoms[:-1]), max_neighbor_per_atom=288) as general:
+        tile.build()
+        general.build()
+        assert tile.counts()["outside_atoms"] == 0 and general.counts()["outside_atoms"] == 1
+        assert tile.counts()["truncated_atoms"] == 0
+        probes = tile.fetch(analysis=False)["probe_pos"]
+        if len(probes):
+            q = np.concatenate([q, probes[:200, :3], probes[:200, :3] + rng.normal(0, 1e-4, (len(probes[:200]), 3)).astype(np.float32)])
+        gq = rng.standard_normal(len(q)).astype(np.float32)
+        gq[plain:] = 0.0  # a gradient is defined where one primitive is nearest
+        got, kind, grad = evaluate(tile, q, gq)
+        want, wkind, wgrad = evaluate(general, q, gq)
+    assert np.array_equal(got, want)
+    assert np.mean(kind == wkind) > 0.999  # equal distances may go by the atoms' order, which the box changes
+    # float32 sums in any order; a probe near the plane of its atoms moves by thousands of their steps
+    assert np.linalg.norm(grad - wgrad) <= 1e-4 * max(np.linalg.norm(wgrad), 1e-6)
+
+
+@pytest.mark.parametrize("m", [1, 2, 31, 32, 33, 127, 2433, 4999, 38913, 77825])
+def test_values_do_not_depend_on_the_tile(m):
+    """Any number of queries, in any order: the same value for each."""
+    atoms = synth.globule(1200, 41)
+    q = synth.queries(atoms, 80000, 42)
+    order = np.random.default_rng(m).permutation(len(q))[:m]
+    with SesBuild(atoms, 1.4, "full") as g:
+        g.build()
+        want, wkind, _ = evaluate(g, q)
+        got, kind, _ = evaluate(g, q[order])
+    assert np.array_equal(got, want[order])
+    assert np.array_equal(kind, wkind[order])
