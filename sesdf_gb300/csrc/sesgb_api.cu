@@ -1004,11 +1004,14 @@ extern "C"
                 return SESGB_ERR_CUDA;
             c->cavBytes = small;
         }
-        double bounds[ 6 ];
-        launch_cavity_bounds( c->b, rp, static_cast<double *>( c->cavMem ), s );
-        if ( !cuda_ok( c, cudaMemcpyAsync( bounds, c->cavMem, sizeof( bounds ), cudaMemcpyDeviceToHost, s ), "bounds" )
+        unsigned long long keys[ 6 ];
+        launch_cavity_bounds( c->b, rp, static_cast<unsigned long long *>( c->cavMem ), s );
+        if ( !cuda_ok( c, cudaMemcpyAsync( keys, c->cavMem, sizeof( keys ), cudaMemcpyDeviceToHost, s ), "bounds" )
              || !cuda_ok( c, cudaStreamSynchronize( s ), "bounds" ) )
             return SESGB_ERR_CUDA;
+        double bounds[ 6 ];
+        for ( int a = 0; a < 6; a++ )
+            bounds[ a ] = cavity_bound( keys[ a ] );
         CavGrid  g;
         uint64_t V = 1;
         for ( int a = 0; a < 3; a++ )
@@ -1032,9 +1035,10 @@ extern "C"
             return SESGB_ERR_TOO_LARGE;
         }
         const uint32_t rootCap = (uint32_t)std::min<uint64_t>( V, 1u << 22 );
-        const size_t   need    = small + ( ( ( V + 31 ) / 32 * 4 + 255 ) & ~(size_t)255 ) + ( ( V * 4 + 255 ) & ~(size_t)255 )
-                            + 2 * ( ( (size_t)rootCap * 4 + 255 ) & ~(size_t)255 ) + ( ( ( rootCap + 1ull ) * 4 + 255 ) & ~(size_t)255 )
-                            + ( ( rootCap + 1ull + 255 ) & ~(size_t)255 ) + radix_scratch_bytes( rootCap ) + 256;
+        const uint64_t words   = ( V + 31 ) / 32;
+        auto           padded  = []( size_t bytes ) { return ( bytes + 255 ) & ~(size_t)255; };
+        const size_t   need    = small + 3 * padded( words * 4 ) + padded( V * 4 ) + padded( ( words + 1 ) * 4 ) + padded( ( rootCap + 1ull ) * 4 )
+                            + padded( rootCap + 1ull ) + scan_scratch_bytes( words ) + 256;
         if ( need > c->cavBytes )
         {
             cudaFree( c->cavMem );
@@ -1044,18 +1048,21 @@ extern "C"
                 return SESGB_ERR_CUDA;
             c->cavBytes = need;
         }
-        char *     p       = static_cast<char *>( c->cavMem );
-        uint32_t * scalars = reinterpret_cast<uint32_t *>( carve( p, small ) );
-        uint32_t * bits    = reinterpret_cast<uint32_t *>( carve( p, ( V + 31 ) / 32 * 4 ) );
-        int32_t *  labels  = reinterpret_cast<int32_t *>( carve( p, V * 4 ) );
-        uint32_t * roots   = reinterpret_cast<uint32_t *>( carve( p, (size_t)rootCap * 4 ) );
-        uint32_t * order   = reinterpret_cast<uint32_t *>( carve( p, (size_t)rootCap * 4 ) );
-        uint32_t * voxels  = reinterpret_cast<uint32_t *>( carve( p, ( rootCap + 1ull ) * 4 ) );
-        uint8_t *  border  = reinterpret_cast<uint8_t *>( carve( p, rootCap + 1ull ) );
-        void *     radix   = carve( p, radix_scratch_bytes( rootCap ) );
-        launch_cavity_labels( c->b, g, bits, labels, roots, rootCap, scalars, s );
-        uint32_t hs[ 2 ];
-        if ( !cuda_ok( c, cudaMemcpyAsync( hs, scalars, sizeof( hs ), cudaMemcpyDeviceToHost, s ), "labels" )
+        char *     p = static_cast<char *>( c->cavMem );
+        CavBuffers cb;
+        cb.scalars   = reinterpret_cast<uint32_t *>( carve( p, small ) );
+        cb.bits      = reinterpret_cast<uint32_t *>( carve( p, words * 4 ) );
+        cb.runs      = reinterpret_cast<uint32_t *>( carve( p, words * 4 ) );
+        cb.rootBits  = reinterpret_cast<uint32_t *>( carve( p, words * 4 ) );
+        cb.labels    = reinterpret_cast<int32_t *>( carve( p, V * 4 ) );
+        cb.rootCount = reinterpret_cast<uint32_t *>( carve( p, ( words + 1 ) * 4 ) );
+        cb.voxels    = reinterpret_cast<uint32_t *>( carve( p, ( rootCap + 1ull ) * 4 ) );
+        cb.border    = reinterpret_cast<uint8_t *>( carve( p, rootCap + 1ull ) );
+        cb.scan      = carve( p, scan_scratch_bytes( words ) );
+        const uint32_t nProbes = device_probe_component ? c->hCounts->I : 0u;
+        launch_cavities( c->b, g, cb, rootCap, c->b.probePos, nProbes, device_probe_component, s );
+        uint32_t hs[ 3 ];
+        if ( !cuda_ok( c, cudaMemcpyAsync( hs, cb.scalars, sizeof( hs ), cudaMemcpyDeviceToHost, s ), "labels" )
              || !cuda_ok( c, cudaStreamSynchronize( s ), "labels" ) )
             return SESGB_ERR_CUDA;
         if ( hs[ 1 ] )
@@ -1063,20 +1070,10 @@ extern "C"
             c->err = ( hs[ 1 ] & 4u ) ? "more than 2^22 components in the cavity grid" : "cavity labelling did not converge";
             return SESGB_ERR_OVERFLOW;
         }
-        const uint32_t nRoots = hs[ 0 ];
-        radix_sort( roots, order, nRoots, 28, radix, s ); // voxel indices are below 2^28
-        const uint32_t nProbes = device_probe_component ? c->hCounts->I : 0u;
-        launch_cavity_relabel( g, labels, roots, nRoots, voxels, border, c->b.probePos, nProbes, device_probe_component, s );
-        std::vector<uint8_t> hb( nRoots + 1ull );
-        if ( !cuda_ok( c, cudaMemcpyAsync( hb.data(), border, hb.size(), cudaMemcpyDeviceToHost, s ), "components" )
-             || !cuda_ok( c, cudaStreamSynchronize( s ), "components" ) )
-            return SESGB_ERR_CUDA;
-        uint32_t ext = 0;
-        for ( uint32_t k = 1; k <= nRoots; k++ )
-            ext += hb[ k ] != 0;
-        c->cavLabels     = labels;
-        c->cavVoxels     = voxels;
-        c->cavBorder     = border;
+        const uint32_t nRoots = hs[ 0 ], ext = hs[ 2 ];
+        c->cavLabels     = cb.labels;
+        c->cavVoxels     = cb.voxels;
+        c->cavBorder     = cb.border;
         c->cavV          = V;
         c->cavComponents = nRoots;
         for ( int a = 0; a < 3; a++ )

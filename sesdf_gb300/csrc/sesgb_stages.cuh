@@ -156,16 +156,25 @@ namespace sesgb
         double   rp;
         uint32_t dims[ 3 ];
     };
-    // out (device double[6]): min and max of c -+ (r + rp) over the build's atoms
-    void launch_cavity_bounds( const Build & b, double rp, double * out, cudaStream_t s );
-    // occupancy bits, union-find labels (root = smallest voxel index), roots collected into roots
-    // (scalars[0] = count, scalars[1] = error bits)
-    void launch_cavity_labels( const Build & b, const CavGrid & g, uint32_t * bits, int32_t * labels, uint32_t * roots,
-                               uint32_t rootCap, uint32_t * scalars, cudaStream_t s );
-    // labels 1..nRoots by the rank of their root in the sorted roots; voxel counts and border flags
-    // per label; the label of each of k probes (probeLabel may be null)
-    void launch_cavity_relabel( const CavGrid & g, int32_t * labels, const uint32_t * roots, uint32_t nRoots, uint32_t * voxels,
-                                uint8_t * border, const float4 * probes, uint32_t k, int32_t * probeLabel, cudaStream_t s );
+    // keys (device, 6): ordered keys of the min and max of c -+ (r + rp) over the build's atoms; cavity_bound: a key's value
+    void   launch_cavity_bounds( const Build & b, double rp, unsigned long long * keys, cudaStream_t s );
+    double cavity_bound( unsigned long long key );
+    struct CavBuffers
+    {
+        uint32_t * bits;      // (V + 31) / 32: occupancy
+        uint32_t * runs;      // (V + 31) / 32: first voxels of the runs of free voxels along z
+        uint32_t * rootBits;  // (V + 31) / 32
+        int32_t *  labels;    // V, in an allocation of a multiple of four
+        uint32_t * rootCount; // (V + 31) / 32 + 1
+        uint32_t * voxels;    // rootCap + 1: voxels of each component
+        uint8_t *  border;    // rootCap + 1: touches the border
+        uint32_t * scalars;   // components, error bits, components that touch the border
+        void *     scan;      // scan_scratch_bytes( (V + 31) / 32 )
+    };
+    // occupancy bits, union-find labels, components 1.. in the order of their first voxel with voxel counts and border
+    // flags, and the label of each of k probes (probeLabel may be null); no host synchronisation
+    void launch_cavities( const Build & b, const CavGrid & g, const CavBuffers & c, uint32_t rootCap, const float4 * probes, uint32_t k,
+                          int32_t * probeLabel, cudaStream_t s );
     // SES area of the primitives of a full-surface build (sesgb_area.cu): parts (device
     // double[3]: convex, toroidal, concave), atomArea (optional, float[n], input order)
     size_t area_scratch_bytes( const Build & b );
