@@ -301,17 +301,24 @@ namespace
             if ( profile )
                 cudaEventRecordWithFlags( c->ev[ k ], s, capturing ? cudaEventRecordExternal : cudaEventRecordDefault );
         };
-        cudaMemsetAsync( d, 0, sizeof( DeviceCounts ), s );
+        const bool small = small_front( b, c->gridBits );
+        if ( !small )
+            cudaMemsetAsync( d, 0, sizeof( DeviceCounts ), s );
         if ( n == 0 )
             return;
 
         // A: reference-grid order, neighbour grid, neighbour lists
         mark( 0 );
-        launch_hash( b, s );
-        radix_sort( b.keys, b.perm, n, c->gridBits, c->radixScratch, s );
-        launch_fine_params( b, -1.f, n, s, b.nbrSpan );
-        launch_gather( b, s );
-        launch_cells( b, 0, n, nullptr, sc, s );
+        if ( small )
+            launch_front( b, c->gridBits, s );
+        else
+        {
+            launch_hash( b, s );
+            radix_sort( b.keys, b.perm, n, c->gridBits, c->radixScratch, s );
+            launch_fine_params( b, -1.f, n, s, b.nbrSpan );
+            launch_gather( b, s );
+            launch_cells( b, 0, n, nullptr, sc, s );
+        }
         mark( 1 );
         launch_neighbors( b, s );
         exclusive_scan( b.nbrCount, b.pairOff, n, nullptr, &d->P, sc, s );
@@ -355,8 +362,13 @@ namespace
         mark( 8 );
         // singular probes are sparse in the atoms' box: their grid stays on cutoff cells (a half-cutoff
         // grid hits the cell capacity and is coarsened; measured slower)
-        launch_fine_params( b, 2.f * c->rp + 0.01f, 0, s, 1 );
-        launch_cells( b, 1, b.capProbes, &d->Q, sc, s );
+        if ( small )
+            launch_front_probes( b, 2.f * c->rp + 0.01f, s );
+        else
+        {
+            launch_fine_params( b, 2.f * c->rp + 0.01f, 0, s, 1 );
+            launch_cells( b, 1, b.capProbes, &d->Q, sc, s );
+        }
         launch_probe_neighbors( b, s );
 
         // H: exterior tori

@@ -2971,7 +2971,7 @@ namespace sesgb
     cudaError_t configure_kernels( const Build & b )
     {
         const size_t vs = vis_smem_per_warp( b.cap ), ps = probe_smem_per_warp( b.cap );
-        cudaError_t  e  = cudaSuccess;
+        cudaError_t  e  = configure_front();
         auto         set = [ & ]( const void * f, size_t bytes ) {
             if ( e == cudaSuccess )
                 e = cudaFuncSetAttribute( f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes );

@@ -128,6 +128,15 @@ namespace sesgb
     void launch_cells( const Build & b, int kind, uint32_t nHost, const uint32_t * nDevice, void * scanScratch,
                        cudaStream_t s );
     void launch_batch_finish( const Build & b, cudaStream_t s );
+    // the head of a small build of one molecule in one block (sesgb_front.cu): counters zeroed, reference-grid order and
+    // neighbour grid; and the grid of its singular probes. Up to 8192 atoms: one SM is then faster than
+    // the general path's launches (a build of 6,007 atoms gains 16 us), at 11,638 atoms it was slower (250 us against 235).
+    constexpr uint32_t kFrontAtoms = 8192;
+    constexpr int      kFrontBits  = 12; // of the reference grid's hash
+    bool        small_front( const Build & b, int bits );
+    void        launch_front( const Build & b, int bits, cudaStream_t s );
+    void        launch_front_probes( const Build & b, float cutoff, cudaStream_t s );
+    cudaError_t configure_front();
     // signed distance to the SES at float3 query points (sesgb_sdf.cu)
     struct SdfState
     {
