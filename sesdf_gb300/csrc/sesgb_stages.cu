@@ -1907,54 +1907,211 @@ namespace sesgb
             }
         }
 
-        // Exact position of one side of a kept probe in double precision, rounded once to
-        // float32; returns the singular flag. Out of line, so that its conversions run
-        // only for the few probes whose float-float position cannot be rounded safely.
-        __device__ __noinline__ bool fill_position_d( float4 ai, float4 aj, float4 ak, float rpf, uint32_t side, float3 & pf )
+        // solve_d with four lanes per triplet: lane c of a group of four works out component c of the vectors (lane 3 repeats
+        // z) and the dots' products are exchanged, so that every operation and its order are solve_d's. An FP64
+        // instruction occupies its pipe for 64 cycles however few lanes use it: a chain of ~70 instead of ~130.
+        // All 32 lanes call it; x1 and x2 are the component of the lane. Out of line, so that its conversions run only where it
+        // is called.
+        __device__ __noinline__ bool solve_d4( float4 ai, float4 aj, float4 ak, float rpf, double & x1, double & x2, double & h2 )
         {
-            const double rp = (double)rpf;
-            d3           x[ 2 ];
-            double       h2 = 0.0;
-            solve_d( D3( ai ), (double)ai.w, D3( aj ), (double)aj.w, D3( ak ), (double)ak.w, rp, x[ 0 ], x[ 1 ], h2 );
-            const d3 xs = side ? x[ 1 ] : x[ 0 ];
-            pf          = make_float3( __double2float_rn( xs.x ), __double2float_rn( xs.y ), __double2float_rn( xs.z ) );
-            return singular_d( h2, rp );
+            constexpr uint32_t kAll = 0xffffffffu;
+            const uint32_t     lane = lane_id(), g = lane & 28u, c = min( lane & 3u, 2u );
+            const uint32_t     g1 = g + ( c + 1u ) % 3u, g2 = g + ( c + 2u ) % 3u;
+            auto comp = [ & ]( const float4 & v ) { return (double)( c == 0u ? v.x : c == 1u ? v.y : v.z ); };
+            auto dot3 = [ & ]( double pr ) {
+                const double y = __shfl_sync( kAll, pr, g + 1u ), z = __shfl_sync( kAll, pr, g + 2u );
+                return __dadd_rn( __dadd_rn( __shfl_sync( kAll, pr, g ), y ), z );
+            };
+            const double R   = __dadd_rn( (double)( c == 0u ? ai.w : c == 1u ? aj.w : ak.w ), (double)rpf );
+            const double RR  = __dmul_rn( R, R );
+            const double Ri2 = __shfl_sync( kAll, RR, g ), Rj2 = __shfl_sync( kAll, RR, g + 1u ), Rk2 = __shfl_sync( kAll, RR, g + 2u );
+            const double ci = comp( ai );
+            const double a = __dsub_rn( comp( aj ), ci ), bv = __dsub_rn( comp( ak ), ci );
+            const double a1 = __shfl_sync( kAll, a, g1 ), a2 = __shfl_sync( kAll, a, g2 );
+            const double b1 = __shfl_sync( kAll, bv, g1 ), b2 = __shfl_sync( kAll, bv, g2 );
+            const double n  = __dsub_rn( __dmul_rn( a1, b2 ), __dmul_rn( a2, b1 ) );
+            const double n1 = __shfl_sync( kAll, n, g1 ), n2 = __shfl_sync( kAll, n, g2 );
+            // lane 1 works out q, the others p
+            const double pa = __dmul_rn( a, a ), pb = __dmul_rn( bv, bv );
+            const double ax = __shfl_sync( kAll, pa, g ), ay = __shfl_sync( kAll, pa, g + 1u ), az = __shfl_sync( kAll, pa, g + 2u );
+            const double bx = __shfl_sync( kAll, pb, g ), by = __shfl_sync( kAll, pb, g + 1u ), bz = __shfl_sync( kAll, pb, g + 2u );
+            const bool   isQ = c == 1u;
+            const double vv  = __dadd_rn( __dadd_rn( isQ ? bx : ax, isQ ? by : ay ), isQ ? bz : az );
+            const double pq  = __dmul_rn( __dsub_rn( __dadd_rn( vv, Ri2 ), isQ ? Rk2 : Rj2 ), 0.5 );
+            const double p = __shfl_sync( kAll, pq, g ), q = __shfl_sync( kAll, pq, g + 1u );
+            const double inv = __ddiv_rn( 1.0, dot3( __dmul_rn( n, n ) ) );
+            const double bn  = __dsub_rn( __dmul_rn( b1, n2 ), __dmul_rn( b2, n1 ) );
+            const double na  = __dsub_rn( __dmul_rn( n1, a2 ), __dmul_rn( n2, a1 ) );
+            const double y0  = __dmul_rn( __dadd_rn( __dmul_rn( bn, p ), __dmul_rn( na, q ) ), inv );
+            h2               = __dsub_rn( Ri2, dot3( __dmul_rn( y0, y0 ) ) );
+            x1 = x2 = 0.0;
+            if ( !( h2 >= 0.0 ) )
+                return false;
+            const double s  = __dsqrt_rn( __dmul_rn( h2, inv ) );
+            const double xc = __dadd_rn( ci, y0 ), ns = __dmul_rn( n, s );
+            x1              = __dadd_rn( xc, ns );
+            x2              = __dsub_rn( xc, ns );
+            return true;
+        }
+
+        // outside atom al's probe-centre sphere, in double precision
+        __device__ __noinline__ bool outside_d( float4 al, double x, double y, double z, float rpf )
+        {
+            const double R = __dadd_rn( (double)al.w, (double)rpf );
+            const d3     v = dsub( D3( al ), D3( x, y, z ) );
+            return __dsub_rn( ddot( v, v ), __dmul_rn( R, R ) ) > 0.0;
+        }
+
+        // occlusion_d with four lanes per triplet, 32 neighbours a step: the same tests on the same numbers. All 32 lanes
+        // call it (have: the group holds a triplet); x1, x2: the lane's component of the points. The count of
+        // double-precision tests is that of a walk in order which ends at the first occluder.
+        __device__ __forceinline__ void occlusion_d4( const Build & b, bool have, uint32_t i, const float4 & ai, uint32_t sj, uint32_t sk,
+                                                      double x1, double x2, bool vis[ 2 ], uint32_t & fp64 )
+        {
+            constexpr uint32_t kAll = 0xffffffffu;
+            const uint32_t     lane = lane_id(), g = lane & 28u, c = lane & 3u;
+            const double       ci = (double)( c == 0u ? ai.x : c == 1u ? ai.y : ai.z );
+            const float        r1 = __double2float_rn( __dsub_rn( x1, ci ) ), r2 = __double2float_rn( __dsub_rn( x2, ci ) );
+            f3                 xr[ 2 ];
+            xr[ 0 ] = F3( __shfl_sync( kAll, r1, g ), __shfl_sync( kAll, r1, g + 1u ), __shfl_sync( kAll, r1, g + 2u ) );
+            xr[ 1 ] = F3( __shfl_sync( kAll, r2, g ), __shfl_sync( kAll, r2, g + 1u ), __shfl_sync( kAll, r2, g + 2u ) );
+            d3 x[ 2 ];
+            x[ 0 ] = D3( __shfl_sync( kAll, x1, g ), __shfl_sync( kAll, x1, g + 1u ), __shfl_sync( kAll, x1, g + 2u ) );
+            x[ 1 ] = D3( __shfl_sync( kAll, x2, g ), __shfl_sync( kAll, x2, g + 1u ), __shfl_sync( kAll, x2, g + 2u ) );
+            const uint32_t   ni  = have ? b.nbrCount[ i ] : 0u;
+            const uint32_t * row = b.nbr + (size_t)( have ? i : 0u ) * b.cap;
+            for ( uint32_t s0 = 0; __any_sync( kAll, s0 < ni && ( vis[ 0 ] || vis[ 1 ] ) ); s0 += 4u * kOccChunk )
+            {
+                uint32_t id[ kOccChunk ];
+                float4   al[ kOccChunk ];
+#pragma unroll
+                for ( uint32_t u = 0; u < kOccChunk; u++ )
+                    id[ u ] = s0 + 4u * u + c < ni ? row[ s0 + 4u * u + c ] : 0u;
+#pragma unroll
+                for ( uint32_t u = 0; u < kOccChunk; u++ )
+                    al[ u ] = b.atoms[ id[ u ] ];
+                uint32_t first[ 2 ] = { 0xffffffffu, 0xffffffffu }; // the lane's first occluder
+                uint32_t exact[ 2 ] = { 0u, 0u };                   // neighbours of the double-precision test, a bit per u
+#pragma unroll
+                for ( uint32_t u = 0; u < kOccChunk; u++ )
+                {
+                    const uint32_t sl = s0 + 4u * u + c;
+                    if ( sl >= ni || sl == sj || sl == sk )
+                        continue;
+                    const f3    dl  = F3( al[ u ].x - ai.x, al[ u ].y - ai.y, al[ u ].z - ai.z );
+                    const float Rl  = al[ u ].w + b.rp;
+                    const float Rl2 = Rl * Rl;
+                    for ( int e = 0; e < 2; e++ )
+                    {
+                        if ( !vis[ e ] || first[ e ] != 0xffffffffu )
+                            continue;
+                        const f3    ev = dl - xr[ e ];
+                        const float ee = dot( ev, ev );
+                        const float m  = ee - Rl2;
+                        const float em = kRel * ( ee + Rl2 + 1.f );
+                        bool        in = m < -em;
+                        if ( !in && !( m > em ) )
+                        {
+                            in = !outside_d( al[ u ], x[ e ].x, x[ e ].y, x[ e ].z, b.rp );
+                            exact[ e ] |= 1u << u;
+                        }
+                        if ( in )
+                            first[ e ] = sl;
+                    }
+                }
+                for ( int e = 0; e < 2; e++ )
+                {
+                    uint32_t f = first[ e ];
+                    f          = min( f, __shfl_xor_sync( kAll, f, 1 ) );
+                    f          = min( f, __shfl_xor_sync( kAll, f, 2 ) );
+                    for ( uint32_t m = exact[ e ]; m; m &= m - 1u )
+                        fp64 += s0 + 4u * ( (uint32_t)__ffs( (int)m ) - 1u ) + c <= f;
+                    vis[ e ] = vis[ e ] && f == 0xffffffffu;
+                }
+            }
         }
 
         // The double-precision pass, one job per thread with full warps: exact
         // probe positions (the solve of findIntersectionsBetweenCircles in IEEE
         // double, rounded once to float32) and the decisions the float32 screen
-        // left open.
-        __global__ void __launch_bounds__( 128 ) k_probe_jobs( Build b )
+        // left open. Bound by the latency of one job's chain at every size of build (27 us at
+        // 2,000 atoms, 39 at 100,000, when a thread took a fill job and then a band job, each a chain of FP64
+        // instructions): the band jobs are taken from the first thread up, the fill jobs from the last warp down, so that
+        // the two chains run side by side and the longer one starts first, and both solve with four lanes per triplet
+        // (solve_d4): 17 us at 2,000 atoms, 33 at 100,000, 146 (as before) at 1,000,000.
+        // Four lanes per job take 2 to 3 times the FP64 cycles in all: from kBandGroups jobs on, where
+        // these and not the chain are the time, a thread takes a band job.
+        constexpr uint32_t kBandGroups = 24576;
+        __global__ void __launch_bounds__( 128, 5 ) k_probe_jobs( Build b )
         {
             pdl_begin();
             const uint32_t nFill = min( b.counts->jobs, b.capProbes );
             const uint32_t nBand = min( b.counts->bandJobs, b.capProbes - nFill );
             const double   rp    = (double)b.rp;
             const uint32_t lane  = lane_id();
+            const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
             uint32_t       fp64 = 0, full64 = 0, ffMiss = 0;
             // fill jobs, one per thread: float-float first, double precision only where
             // the float-float result cannot decide
-            for ( uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nFill; t += gridDim.x * blockDim.x )
+            // (whole warps: the lanes work together on what float-float leaves open)
+            for ( uint32_t t0 = threads - 32u - ( tid - lane ); t0 < nFill; t0 += threads )
             {
-                const uint4    jb   = b.jobs[ t ];
+                const uint32_t t  = t0 + lane;
+                uint4          jb = make_uint4( 0u, 0xffffffffu, 0u, 0u );
+                if ( t < nFill )
+                    jb = b.jobs[ t ];
                 const uint32_t ent  = jb.x, i = jb.y;
                 const uint32_t sj   = jb.z & 0xffffu, sk = jb.z >> 16;
                 const uint32_t side = ( jb.w >> 16 ) & 0xffu;
                 // the empty jobs of an atom whose entries did not fit (a build that is redone larger)
-                if ( i >= b.n || ent >= b.capProbes || sj >= b.cap || sk >= b.cap )
-                    continue;
-                const size_t   row  = (size_t)i * b.cap;
-                const float4   ai = b.atoms[ i ], aj = b.atoms[ b.nbr[ row + sj ] ], ak = b.atoms[ b.nbr[ row + sk ] ];
-                int4           cid  = b.stageCid[ ent ];
-                int            aw   = cid.w < 0 ? -cid.w : cid.w;
-                float3         pf;
-                bool           sing = false;
-                if ( !solve_ff( ai, aj, ak, b.rp, side, aw == 3, pf, sing ) )
+                const bool     job = i < b.n && ent < b.capProbes && sj < b.cap && sk < b.cap;
+                float4         ai = make_float4( 0.f, 0.f, 0.f, 0.f ), aj = ai, ak = ai;
+                int4           cid = make_int4( 0, 0, 0, 0 );
+                int            aw  = 0;
+                float3         pf  = make_float3( 0.f, 0.f, 0.f );
+                bool           sing = false, miss = false;
+                if ( job )
                 {
-                    ffMiss++;
-                    sing = fill_position_d( ai, aj, ak, b.rp, side, pf );
+                    const size_t row = (size_t)i * b.cap;
+                    ai               = b.atoms[ i ];
+                    aj               = b.atoms[ b.nbr[ row + sj ] ];
+                    ak               = b.atoms[ b.nbr[ row + sk ] ];
+                    cid              = b.stageCid[ ent ];
+                    aw               = cid.w < 0 ? -cid.w : cid.w;
+                    miss             = !solve_ff( ai, aj, ak, b.rp, side, aw == 3, pf, sing );
+                    ffMiss += miss;
                 }
+                // float-float could not decide: eight at a time, four lanes each, in double precision, rounded once
+                for ( uint32_t mm = __ballot_sync( 0xffffffffu, miss ); mm; )
+                {
+                    uint32_t m = mm;
+                    for ( uint32_t k = 0; k < ( lane >> 2 ); k++ )
+                        m &= m - 1u;
+                    const uint32_t src = m ? (uint32_t)__ffs( (int)m ) - 1u : 0u;
+                    auto           from = [ & ]( const float4 & v ) {
+                        return make_float4( __shfl_sync( 0xffffffffu, v.x, src ), __shfl_sync( 0xffffffffu, v.y, src ),
+                                                      __shfl_sync( 0xffffffffu, v.z, src ), __shfl_sync( 0xffffffffu, v.w, src ) );
+                    };
+                    const float4   bi = from( ai ), bj = from( aj ), bk = from( ak );
+                    const uint32_t bs = __shfl_sync( 0xffffffffu, side, src );
+                    double         x1, x2, h2;
+                    solve_d4( bi, bj, bk, b.rp, x1, x2, h2 );
+                    const float    f    = __double2float_rn( bs ? x2 : x1 );
+                    const bool     sg   = singular_d( h2, rp );
+                    const uint32_t rank = __popc( mm & lanemask_lt() ), at = 4u * min( rank, 7u );
+                    const float    fx = __shfl_sync( 0xffffffffu, f, at ), fy = __shfl_sync( 0xffffffffu, f, at + 1u ),
+                                fz = __shfl_sync( 0xffffffffu, f, at + 2u );
+                    const bool     fs = __shfl_sync( 0xffffffffu, (int)sg, at ) != 0;
+                    if ( ( ( mm >> lane ) & 1u ) && rank < 8u )
+                    {
+                        pf   = make_float3( fx, fy, fz );
+                        sing = fs;
+                    }
+                    for ( int k = 0; k < 8; k++ )
+                        mm &= mm - 1u; // (0 stays 0)
+                }
+                if ( !job )
+                    continue;
                 if ( aw == 3 )
                 {
                     aw                = sing ? 2 : 1;
@@ -1964,9 +2121,52 @@ namespace sesgb
                 }
                 b.stagePos[ ent ] = make_float4( pf.x, pf.y, pf.z, (float)cid.w );
             }
-            // band candidates, one per thread (the double-precision solve, occlusion and
-            // singular test), stored from the top of the job array
-            for ( uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < nBand; g += gridDim.x * blockDim.x )
+            __syncwarp();
+            // band candidates (the double-precision solve, occlusion and singular test), stored from the top of the
+            // job array: four lanes each
+            if ( nBand <= kBandGroups )
+            {
+                for ( uint32_t g0 = ( tid - lane ) >> 2; g0 < nBand; g0 += threads >> 2 )
+                {
+                    const uint32_t g  = g0 + ( lane >> 2 );
+                    uint4          jb = make_uint4( 0u, 0xffffffffu, 0u, 0u );
+                    if ( g < nBand )
+                        jb = b.jobs[ b.capProbes - 1u - g ];
+                    const uint32_t ent = jb.x, i = jb.y;
+                    const uint32_t sj  = jb.z & 0xffffu, sk = jb.z >> 16;
+                    bool           job = i < b.n && ent + 1u < b.capProbes && sj < b.cap && sk < b.cap;
+                    float4         ai = make_float4( 0.f, 0.f, 0.f, 0.f ), aj = ai, ak = ai;
+                    if ( job )
+                    {
+                        const size_t row = (size_t)i * b.cap;
+                        ai               = b.atoms[ i ];
+                        aj               = b.atoms[ b.nbr[ row + sj ] ];
+                        ak               = b.atoms[ b.nbr[ row + sk ] ];
+                    }
+                    double x1, x2, h2;
+                    full64 += job && ( lane & 3u ) == 0u;
+                    const bool ok = solve_d4( ai, aj, ak, b.rp, x1, x2, h2 );
+                    job           = job && ok;
+                    bool vis[ 2 ] = { job, job };
+                    occlusion_d4( b, job, i, ai, sj, sk, x1, x2, vis, fp64 );
+                    const int   aw = singular_d( h2, rp ) ? 2 : 1;
+                    const float f1 = __double2float_rn( x1 ), f2 = __double2float_rn( x2 );
+                    for ( int e = 0; e < 2; e++ )
+                    {
+                        const float  f  = e == 0 ? f1 : f2;
+                        const float  fy = __shfl_down_sync( 0xffffffffu, f, 1 ), fz = __shfl_down_sync( 0xffffffffu, f, 2 );
+                        if ( !vis[ e ] || ( lane & 3u ) )
+                            continue;
+                        const int w = e == 0 ? aw : -aw;
+                        b.stageCid[ ent + e ].w = w;
+                        b.stagePos[ ent + e ]   = make_float4( f, fy, fz, (float)w );
+                        atomicAdd( aw == 2 ? &b.singCnt[ i ] : &b.regCnt[ i ], 1u );
+                    }
+                    __syncwarp();
+                }
+            }
+            else
+            for ( uint32_t g = tid; g < nBand; g += threads )
             {
                 const uint4    jb  = b.jobs[ b.capProbes - 1u - g ];
                 const uint32_t ent = jb.x, i = jb.y;
