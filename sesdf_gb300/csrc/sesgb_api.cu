@@ -60,6 +60,7 @@ struct sesgb_ctx
     DeviceCounts * hCounts = nullptr;
     void *         scanScratch = nullptr;
     size_t         scanScratchBytes = 0;
+    void *         cellScratch = nullptr; // of the singular probes' cells
     void *         radixScratch = nullptr;
     uint32_t *     g2t = nullptr;
 
@@ -273,6 +274,7 @@ namespace
         const uint64_t scanMax = std::max<uint64_t>( { (uint64_t)c->n + 1, C1 + 1, (uint64_t)b.capCells + 1 } );
         c->scanScratchBytes    = scan_scratch_bytes( scanMax );
         c->scanScratch         = dalloc<char>( c, L, c->scanScratchBytes, ok );
+        c->cellScratch         = dalloc<char>( c, L, scan_scratch_bytes( (uint64_t)b.capCells + 1 ), ok );
         return ok;
     }
 
@@ -289,8 +291,13 @@ namespace
     const char * kStageNames[] = { "grid",       "neighbors", "visibility", "circles",         "probes",
                                    "probe_jobs", "place",     "segments",   "probe_neighbors", "tori" };
 
-    // all launches of one build; no host synchronisation inside
-    void enqueue( sesgb_ctx * c, cudaStream_t s, bool profile, bool capturing = false )
+    // all launches of one build; no host synchronisation inside. side: a second stream of a capture, on which the
+    // singular probes' neighbours become a branch of the graph beside the segments or tori (both read the placed probes,
+    // neither what the other writes; the branch has its own scan scratch). Both are latency chains of small kernels: a build
+    // of 2,000 atoms takes 136 us instead of 146, an exterior one of 11,638 atoms 211 instead of 225, of 100,000 atoms 792
+    // instead of 806; at 1,000,000, where each fills the GPU, 6691 instead of 6692.
+    void enqueue( sesgb_ctx * c, cudaStream_t s, bool profile, bool capturing = false, cudaStream_t side = nullptr,
+                  const cudaEvent_t * sideEvents = nullptr )
     {
         Build &     b    = c->b;
         const auto  n    = c->n;
@@ -347,6 +354,12 @@ namespace
         launch_zero2( b.ccount, b.ccursor, b.capC1, &d->C1, s ); // per-circle probe counts and list cursors
         launch_place( b, s );
         mark( 7 );
+        const cudaStream_t sp = side ? side : s; // the stream of the probes' neighbours
+        if ( side )
+        {
+            cudaEventRecord( sideEvents[ 0 ], s );
+            cudaStreamWaitEvent( side, sideEvents[ 0 ], 0 );
+        }
 
         // F: segments
         if ( c->mode == SESGB_MODE_FULL )
@@ -363,13 +376,13 @@ namespace
         // singular probes are sparse in the atoms' box: their grid stays on cutoff cells (a half-cutoff
         // grid hits the cell capacity and is coarsened; measured slower)
         if ( small )
-            launch_front_probes( b, 2.f * c->rp + 0.01f, s );
+            launch_front_probes( b, 2.f * c->rp + 0.01f, sp );
         else
         {
-            launch_fine_params( b, 2.f * c->rp + 0.01f, 0, s, 1 );
-            launch_cells( b, 1, b.capProbes, &d->Q, sc, s );
+            launch_fine_params( b, 2.f * c->rp + 0.01f, 0, sp, 1 );
+            launch_cells( b, 1, b.capProbes, &d->Q, c->cellScratch, sp );
         }
-        launch_probe_neighbors( b, s );
+        launch_probe_neighbors( b, sp );
 
         // H: exterior tori
         mark( 9 );
@@ -378,6 +391,11 @@ namespace
             launch_tori( b, s );
             exclusive_scan( b.torCnt, b.torOff, n, nullptr, &d->T, sc, s );
             launch_tori_emit( b, s );
+        }
+        if ( side )
+        {
+            cudaEventRecord( sideEvents[ 1 ], side );
+            cudaStreamWaitEvent( s, sideEvents[ 1 ], 0 );
         }
         // batches: per-molecule records, molecule-local ids
         launch_batch_finish( b, s );
@@ -468,16 +486,33 @@ namespace
             {
                 replayed = false; // the capture counted this build's kernels already
                 const uint64_t l0 = launch_count();
-                cudaStream_t cap;
-                if ( !cuda_ok( c, cudaStreamCreateWithFlags( &cap, cudaStreamNonBlocking ), "stream" ) )
+                cudaStream_t cap = nullptr, side = nullptr;
+                cudaEvent_t  ev[ 2 ] = {};
+                const bool   ok  = cuda_ok( c, cudaStreamCreateWithFlags( &cap, cudaStreamNonBlocking ), "stream" )
+                                && cuda_ok( c, cudaStreamCreateWithFlags( &side, cudaStreamNonBlocking ), "stream" )
+                                && cuda_ok( c, cudaEventCreateWithFlags( &ev[ 0 ], cudaEventDisableTiming ), "event" )
+                                && cuda_ok( c, cudaEventCreateWithFlags( &ev[ 1 ], cudaEventDisableTiming ), "event" );
+                auto         release = [ & ] {
+                    for ( cudaEvent_t e : ev )
+                        if ( e )
+                            cudaEventDestroy( e );
+                    for ( cudaStream_t t : { cap, side } )
+                        if ( t )
+                            cudaStreamDestroy( t );
+                };
+                if ( !ok )
+                {
+                    release();
                     return SESGB_ERR_CUDA;
+                }
                 cudaStreamBeginCapture( cap, cudaStreamCaptureModeThreadLocal );
-                enqueue( c, cap, profile, true ); // stage events become event-record nodes of the graph
+                // stage events become event-record nodes of the graph, the stages then in a row
+                enqueue( c, cap, profile, true, profile ? nullptr : side, ev );
                 cudaMemcpyAsync( c->hCounts, c->b.counts, sizeof( DeviceCounts ), cudaMemcpyDeviceToHost, cap );
                 if ( c->nMol > 1 )
                     cudaMemcpyAsync( c->hMol, c->b.molCounts, sizeof( uint32_t ) * c->nMol * kMolFields, cudaMemcpyDeviceToHost, cap );
                 const cudaError_t e = cudaStreamEndCapture( cap, &c->graph );
-                cudaStreamDestroy( cap );
+                release();
                 if ( !cuda_ok( c, e, "capture" ) )
                     return SESGB_ERR_CUDA;
                 if ( !cuda_ok( c, cudaGraphInstantiate( &c->graphExec, c->graph, 0 ), "instantiate" ) )

@@ -4,6 +4,7 @@ coarsened to the counters), atoms outside the reference grid, and both modes; bu
 import numpy as np
 import pytest
 
+import canon
 from sesdf_gb300 import SesBatch, SesBuild, synth
 from test_gpu_batch import compare
 
@@ -36,18 +37,26 @@ def test_front_matches_general(name, mode):
         compare(g, mols, mode)
 
 
-@pytest.mark.parametrize("n", [700, 5000])
-def test_moved_atoms_and_replay(n):
-    # the recorded build sees new positions (and other radii) on each pass, some outside the grid of the first ones
+@pytest.mark.parametrize("mode", ["full", "exterior"])
+@pytest.mark.parametrize("n", [700, 5000, 12000])
+def test_moved_atoms_and_replay(n, mode):
+    # the recorded build (with the probes' neighbours beside the segments or tori) sees new positions and other
+    # radii on each pass, some outside the grid of the first ones
     a, b = synth.globule(n, 71), synth.globule(n, 72)
     b[:, 3] *= 1.1
     b[:5, :3] += 40.0
-    with SesBuild(a, 1.4, "full") as g, SesBuild(a, 1.4, "full", graph=False) as h:
+    names = ["atoms", "perm", "probe_pos", "probe_ids"]
+    names += ["sectors", "segments"] if mode == "full" else ["tori_pos", "tori_axis", "tori_vs"]
+    with SesBuild(a, 1.4, mode) as g, SesBuild(a, 1.4, mode, graph=False) as h:
         for atoms in (a, b, a):
             out = []
             for k in (g, h):
                 k.set_atoms(atoms)
                 k.build()
                 out.append(k.fetch(analysis=True))
-            for k in ("atoms", "perm", "probe_pos", "probe_ids", "sectors", "segments"):
-                assert np.array_equal(out[0][k], out[1][k], equal_nan=True), k
+            x, y = out
+            for k in names:
+                assert np.array_equal(x[k], y[k], equal_nan=True), k
+            q = x["counts"]["singular_probes"]
+            assert np.array_equal(canon.written_probe_nbrs(x["probe_nbrs"], x["probe_ids"], q),
+                                  canon.written_probe_nbrs(y["probe_nbrs"], y["probe_ids"], q))
