@@ -47,7 +47,7 @@ namespace sesgb
             const float4 *   pos;     // atom (x, y, z, r; r < 0 without accessible surface), probe (x, y, z, 0), arc ball (centre, radius)
             const uint32_t * id;      // sorted atom (bit 31: no accessible direction), probe, arc, query
             const uint2 *    arcs;    // circle (i, j), i < j, of every arc
-            const uint32_t * open;    // per sorted atom: 256 bins of directions, those that may be accessible (direction_bin)
+            const uint32_t * open;    // per sorted atom: 256 bins of directions, those that may be accessible (direction_bin); null without arcs
             const uint32_t * flags;   // [0] arcs, [1] queries listed for the general search, [2] 1: the arcs did not fit
         };
 
@@ -947,7 +947,7 @@ namespace sesgb
                         p.w = -p.w;
                         own |= 0x80000000u;
                     }
-                    else
+                    else if ( ix.open )
                     {
                         const uint4 * o = reinterpret_cast<const uint4 *>( ix.open ) + 2u * (size_t)t;
                         const uint4   u = o[ 0 ], v = o[ 1 ];
@@ -1924,19 +1924,20 @@ namespace sesgb
             }
         }
 
-        // the listed queries by the general search, a warp each
+        // the listed queries (without a list: all m, in cell order) by the general search, a warp each; six blocks a SM: 1M
+        // atoms, 40,000 queries 5221 us (5764 with four, 4774 with eight, whose spills cost a lone query 13 %)
         template<bool kBackward>
-        __global__ void __launch_bounds__( 32 * kSdfWarps ) k_sdf_exact( Build b, SdfIndex ix, const float * queries, float band, float * sdf,
+        __global__ void __launch_bounds__( 32 * kSdfWarps, 6 ) k_sdf_exact( Build b, SdfIndex ix, const float * queries, float band, float * sdf,
                                                                       const float * gradSdf, float * gradSorted, int * kind,
-                                                                      const uint32_t * list, const uint32_t * listCount )
+                                                                      const uint32_t * list, const uint32_t * listCount, uint32_t m )
         {
             __shared__ SdfSmem smem[ kSdfWarps ];
             const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
-            const uint32_t     count = *listCount;
+            const uint32_t     count = list ? *listCount : m;
             uint32_t           overflow = 0;
             for ( uint32_t e = blockIdx.x * kSdfWarps + warp; e < count; e += gridDim.x * kSdfWarps )
             {
-                const uint32_t qi = list[ e ];
+                const uint32_t qi = list ? list[ e ] : ix.id[ ix.start[ 3u * ix.grid.cells ] + e ];
                 const float3 x = make_float3( queries[ 3 * (size_t)qi ], queries[ 3 * (size_t)qi + 1 ], queries[ 3 * (size_t)qi + 2 ] );
                 const SdfHit h = sdf_query( b, ix, x, smem[ warp ], band, overflow );
                 if ( lane == 0 )
@@ -2204,9 +2205,9 @@ namespace sesgb
             return L;
         }
 
-        // Builds the index in scratch: 5 launches for any number of atoms and queries (the grid and the query
+        // Builds the index in scratch (arcs: for the tile search): 5 launches for any number of atoms and queries (the grid and the query
         // order were 17, with a radix sort of the queries)
-        SdfIndex build_index( const Build & b, const SdfState & st, const float * queries, uint32_t m, bool quarters, float band,
+        SdfIndex build_index( const Build & b, const SdfState & st, const float * queries, uint32_t m, bool arcs, bool quarters, float band,
                               void * scratch, uint32_t *& list, uint32_t *& flags, cudaStream_t s )
         {
             SdfIndex ix;
@@ -2232,9 +2233,9 @@ namespace sesgb
             ix.id      = it.id;
             ix.arcs    = reinterpret_cast<uint2 *>( p + L.arcs );
             ix.flags   = flags;
-            ix.open    = reinterpret_cast<uint32_t *>( p + L.open );
+            ix.open    = arcs ? reinterpret_cast<uint32_t *>( p + L.open ) : nullptr;
             cudaMemsetAsync( p + L.flags, 0, L.start - L.flags, s );
-            if ( b.n )
+            if ( b.n && arcs )
                 k_sdf_arcs<<<blocks_of( b.n, kArcWarps ), 32 * kArcWarps, 0, s>>>( b, reinterpret_cast<float4 *>( p + L.balls ),
                                                                                   reinterpret_cast<uint2 *>( p + L.arcs ), it.capArcs,
                                                                                   reinterpret_cast<uint32_t *>( p + L.open ), quarters, flags );
@@ -2242,18 +2243,54 @@ namespace sesgb
             k_sdf_bin<false><<<blocks, 256, 0, s>>>( b, ix, it );
             exclusive_scan( it.count, start, (uint64_t)ix.grid.cells * ( 3u + ix.sub ), nullptr, nullptr, p + L.scan, s );
             k_sdf_bin<true><<<blocks, 256, 0, s>>>( b, ix, it );
-            count_launches( 3 );
+            count_launches( arcs ? 3 : 2 );
             return ix;
         }
 
-        // Lanes per query: one where the queries alone fill the GPU and a tile of 32 stays compact,
-        // more for few or sparse queries
-        uint32_t lanes_per_query( uint32_t m )
+        // Lanes per query. Few queries per atom make the tile of a warp wide, so that its lists are long, and few queries
+        // leave the GPU idle; more lanes per query make the tile smaller and the walk over its lists shorter, and cost
+        // the tile's own work again. Measured over 2,000 to 100,000 atoms and 1,000 to 1,000,000 queries in the molecule's
+        // box, the best G falls with m^(2/3) and grows with n^(1/3): 20,000 atoms with 20,000 queries 349 us at G = 16 (377
+        // at 8, 353 at 32), with 200,000 queries 850 us at G = 4 (890 at 2, 939 at 8, 1123 at 1); 100,000 atoms with 200,000 queries
+        // 1867 us at 8 (2009 at 4, 1952 at 16). One lane from a million queries on: 2,000 atoms 1085 us at
+        // 1, 1145 at 2; 500,000 queries 805 and 612.
+        uint32_t lanes_per_query( uint32_t m, uint32_t n )
         {
-            uint32_t G = 1;
-            while ( G < 32u && (uint64_t)m * G < 32u * 152u * 16u )
+            uint32_t G = m < 1u << 20 ? 2u : 1u;
+            while ( G < 32u && (double)m * m * G * G * G < 3.2e7 * (double)n )
                 G *= 2u;
             return G;
+        }
+        // the arcs' bins in quarters: worth their pass from about four queries per atom on (20,000 atoms: 60,000 queries 522 us
+        // without and 528 with them, 200,000 queries 913 and 850)
+        bool quarters_pay( uint32_t m, uint32_t n ) { return m >= 4u * (uint64_t)n; }
+        // The general search alone, without arcs and tiles: one or a few queries, and few for the size of a large
+        // molecule, whose arcs cost 5.8 us per 1000 atoms whether or not a query comes near them. Queries near the
+        // surface, by the general search and by tiles: 100,000 atoms, 1000 queries 551 and 666 us, 20,000 queries 1850
+        // and 916; 300,000 atoms, 6000 queries 1076 and 1890, 20,000 queries 2526 and 2095; 20,000 atoms, 1 query 96 and 173,
+        // 4 queries 252 and 178.
+        bool general_only( uint32_t m, uint32_t n ) { return 12500ull * m <= n || 20ull * m + 52000u < n; }
+
+        template<bool kBackward>
+        void launch_search( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,
+                            const float * gradSdf, float * gradSorted, void * scratch, cudaStream_t s )
+        {
+            const uint32_t exactBlocks = std::min( blocks_of( m, kSdfWarps ), 152u * 8u );
+            uint32_t *     list, *flags;
+            if ( general_only( m, b.n ) )
+            {
+                const SdfIndex ix = build_index( b, st, queries, m, false, false, band, scratch, list, flags, s );
+                k_sdf_exact<kBackward><<<blocks_of( m, kSdfWarps ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, nullptr,
+                                                                              nullptr, m );
+                count_launches( 1 );
+                return;
+            }
+            const SdfIndex ix = build_index( b, st, queries, m, true, quarters_pay( m, b.n ), band, scratch, list, flags, s );
+            const uint32_t G  = lanes_per_query( m, b.n );
+            k_sdf_tile<kBackward><<<blocks_of( (uint64_t)m * G, 32 * kSdfWarps ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, G, sdf, gradSdf,
+                                                                                                          gradSorted, kind, list, flags + 1 );
+            k_sdf_exact<kBackward><<<exactBlocks, 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, list, flags + 1, m );
+            count_launches( 2 );
         }
     } // namespace
 
@@ -2268,16 +2305,8 @@ namespace sesgb
     void launch_sdf( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,
                      void * scratch, cudaStream_t s )
     {
-        if ( !m )
-            return;
-        uint32_t *     list, *flags;
-        const SdfIndex ix = build_index( b, st, queries, m, m >= 8u * b.n, band, scratch, list, flags, s );
-        const uint32_t G  = lanes_per_query( m );
-        k_sdf_tile<false><<<blocks_of( (uint64_t)m * G, 32 * kSdfWarps ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, G, sdf, nullptr,
-                                                                                                 nullptr, kind, list, flags + 1 );
-        k_sdf_exact<false><<<std::min( blocks_of( m, kSdfWarps ), 152u * 8u ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, nullptr,
-                                                                                                      nullptr, kind, list, flags + 1 );
-        count_launches( 2 );
+        if ( m )
+            launch_search<false>( b, st, queries, m, band, sdf, kind, nullptr, nullptr, scratch, s );
     }
 
     void launch_trace( const Build & b, const SdfState & st, const TraceParams & p, float band, float * depth, float * normals,
@@ -2287,7 +2316,7 @@ namespace sesgb
         if ( !tiles )
             return;
         uint32_t *     list, *flags;
-        const SdfIndex ix = build_index( b, st, nullptr, 0, (uint64_t)p.width * p.height >= b.n, band, scratch, list, flags, s );
+        const SdfIndex ix = build_index( b, st, nullptr, 0, true, (uint64_t)p.width * p.height >= b.n, band, scratch, list, flags, s );
         k_trace<<<(uint32_t)std::min<uint64_t>( blocks_of( tiles, kSdfWarps ), 152u * 64u ), 32 * kSdfWarps, 0, s>>>( b, ix, p, band, depth,
                                                                                                                      normals );
         count_launches( 1 );
@@ -2298,16 +2327,7 @@ namespace sesgb
     {
         cudaMemsetAsync( gradSorted, 0, sizeof( float ) * 4 * (size_t)b.n, s );
         if ( m )
-        {
-            uint32_t *     list, *flags;
-            const SdfIndex ix = build_index( b, st, queries, m, m >= 8u * b.n, band, scratch, list, flags, s );
-            const uint32_t G  = lanes_per_query( m );
-            k_sdf_tile<true><<<blocks_of( (uint64_t)m * G, 32 * kSdfWarps ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, G, nullptr,
-                                                                                                    gradSdf, gradSorted, nullptr, list, flags + 1 );
-            k_sdf_exact<true><<<std::min( blocks_of( m, kSdfWarps ), 152u * 8u ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, nullptr, gradSdf,
-                                                                                                         gradSorted, nullptr, list, flags + 1 );
-            count_launches( 2 );
-        }
+            launch_search<true>( b, st, queries, m, band, nullptr, nullptr, gradSdf, gradSorted, scratch, s );
         if ( b.n )
         {
             k_sdf_unsort<<<blocks_of( b.n, 256 ), 256, 0, s>>>( b, gradSorted, gradInput );

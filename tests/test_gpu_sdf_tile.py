@@ -89,3 +89,34 @@ def test_values_do_not_depend_on_the_tile(m):
         got, kind, _ = evaluate(g, q[order])
     assert np.array_equal(got, want[order])
     assert np.array_equal(kind, wkind[order])
+
+
+@pytest.mark.parametrize("n,few", [(20000, 1), (50000, 4), (60000, 300), (100000, 2000)])
+def test_few_queries_alone_as_among_many(n, few):
+    import torch
+    # few queries take the general search alone, many take tiles: the same bits for each query, and the same
+    # gradient up to the order of its sums where the others have no weight
+    atoms = synth.globule(n, 4200 + few)
+    rng = np.random.default_rng(few)
+    many = 8000
+    k = rng.integers(0, n, many)
+    d = rng.normal(size=(many, 3))
+    q = atoms[k, :3] + d / np.linalg.norm(d, axis=1)[:, None] * (atoms[k, 3:] + rng.uniform(-0.5, 1.5, (many, 1)))
+    q[1::97] += 500.0  # out of reach
+    q = torch.tensor(q.astype(np.float32), device="cuda")
+    w = torch.zeros(many, device="cuda")
+    w[:few] = torch.rand(few, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    out, kind, grad = {}, {}, {}
+    with SesBuild(atoms, 1.4, "full") as g:
+        g.build()
+        for m in (few, many):
+            out[m] = torch.empty(m, device="cuda")
+            kind[m] = torch.empty(m, dtype=torch.int32, device="cuda")
+            grad[m] = torch.empty(n, 4, device="cuda")
+            g.sdf(q.data_ptr(), m, out[m].data_ptr(), kind[m].data_ptr(), s)
+            g.sdf_backward(q.data_ptr(), m, w.data_ptr(), grad[m].data_ptr(), s)
+        torch.cuda.synchronize()
+    assert torch.equal(out[few], out[many][:few]) and torch.equal(kind[few], kind[many][:few])
+    # one query adds to a row once; a row sums at most `few` terms of size at most 1
+    assert torch.allclose(grad[few], grad[many], rtol=0, atol=few * 2.0 ** -22)
