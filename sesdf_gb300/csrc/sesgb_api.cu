@@ -283,6 +283,7 @@ namespace
             b.segments    = L.take<uint4>( b.capSeg );
             b.visBand     = L.take<uint2>( b.capVisBand );
             b.touch       = L.take<uint64_t>( b.capPairs );
+            b.touchHigh   = L.take<uint64_t>( b.capPairs );
             b.torPos      = L.take<float4>( b.capTori );
             b.torAxis     = L.take<float4>( b.capTori );
             b.torVs       = L.take<float4>( b.capTori );

@@ -462,7 +462,8 @@ namespace sesgb
         // queue that k_visibility_band decides in double precision with full
         // warps; k_visibility_final turns the flags into statuses and counts.
         constexpr int kVisQueue   = 128;            // band tests a warp holds before they go to the global queue
-        constexpr int kMaskSlots  = 64;             // atoms with at most this many neighbours keep touch masks
+        constexpr int kMaskSlots  = 64;             // atoms with at most this many neighbours keep touch masks in shared memory
+        constexpr int kWideSlots  = 128;            // atoms with at most this many have touch masks
 
         // status flags between the three visibility kernels
         enum : uint8_t
@@ -614,12 +615,11 @@ namespace sesgb
                 atomicOr( &b.counts->overflow, (uint32_t)kOverflowVisBand );
         }
 
-        struct UnitStride
-        {
-        };
-        __device__ __forceinline__ uint32_t operator*( UnitStride, uint32_t u ) { return u; }
-
         // W warps (atoms) per block; one by default, as k_probes: a slot is freed when its atom is done
+        // Steps of 17 to 20 circles go as 16 and the rest: two lanes and eight lanes a circle for ni / 2 + ni / 8 tests
+        // instead of ni (300,000 atoms: 503.7 us, 506.1 without; up to 24 circles 506.3, up to 31 520.6, a step's own
+        // work being worth more tests than that).
+        constexpr uint32_t kVisSplit = 20;
         template<int W>
         __global__ void __launch_bounds__( 32 * W, 32 / W ) k_visibility( Build b )
         {
@@ -690,38 +690,42 @@ namespace sesgb
             uint32_t nq = 0;
             // Circles go 32 at a time, one per lane, each lane looping over all k
             // (the same k in every lane: shared-memory broadcasts). A last step with
-            // at most 16 circles spreads the k of each circle over a group of G lanes
-            // (k = lane in group + G u). (Steps of 8 or 16 circles with every lane
-            // busy, instead of one step with idle lanes, measured slower on GB300.)
+            // at most 16 circles spreads the k of each circle over a group of G lanes, each a
+            // run of U (the masks of the lanes then only shift into place: 506 us for 300,000 atoms, 520 with
+            // every G-th k per lane).
             for ( uint32_t c0 = 0; c0 < nc; )
             {
-                const uint32_t rem = nc - c0;
-                uint32_t       G   = 1;
+                uint32_t rem = nc - c0;
+                if ( rem > 16 && rem <= kVisSplit )
+                    rem = 16;
+                uint32_t G = 1;
                 if ( rem < 32 )
                     while ( rem * G * 2 <= 32 )
                         G <<= 1;
+                if ( ni > (uint32_t)kMaskSlots && G == 1 )
+                    G = 2; // up to 64 tests a lane: one word of touch bits
                 const uint32_t grp = lane / G, gl = lane % G;
                 const uint32_t gmask = ( G == 32 ? 0xffffffffu : ( ( 1u << G ) - 1u ) ) << ( grp * G );
                 const uint32_t ci    = c0 + grp;
                 const bool     valid = grp < 32 / G && ci < nc;
                 const uint32_t s     = m.list[ valid ? ci : c0 ];
                 const uint32_t U     = ( ni + G - 1 ) / G; // tests per lane
+                const uint32_t first = gl * U;             // of its slots
                 bool           bur = false, tch = false;
-                uint32_t       und[ 2 ] = { 0, 0 }, tou[ 2 ] = { 0, 0 }; // bit u of word w: k = gl + G (32 w + u)
+                uint32_t       und[ 2 ] = { 0, 0 }, tou[ 2 ] = { 0, 0 }; // bit u of word w: k = first + 32 w + u
                 {
                     const VisCircle v = vis_circle( Ri, Mc, theta, m.rel[ s ], m.dd[ s ] );
                     for ( uint32_t u0 = 0; u0 < U; u0 += 32 )
                     {
                         const uint32_t uN = U - u0 < 32 ? U - u0 : 32;
-                        const float4 * qp = m.rel + gl + G * u0;
-                        const float *  dp = m.dd + gl + G * u0;
+                        const float4 * qp = m.rel + first + u0;
+                        const float *  dp = m.dd + first + u0;
                         uint32_t       uw = 0, tw = 0, bw = 0;
-                        auto           run = [ & ]( auto stride ) {
 #pragma unroll 8
                         for ( uint32_t u = 0; u < uN; u++ )
                         {
-                            const float4 q  = qp[ stride * u ];
-                            const float  dk = dp[ stride * u ];
+                            const float4 q  = qp[ u ];
+                            const float  dk = dp[ u ];
                             const float  g  = v.dj.x * q.x + v.dj.y * q.y + v.dj.z * q.z;
                             const float  A  = fmaf( v.m2t, g, q.w );
                             const float  p2 = fmaf( -g * v.inv, g, dk );
@@ -738,11 +742,6 @@ namespace sesgb
                             tw                = __funnelshift_l( ab | gb, tw, 1 );  // A < 0 or G2 < 0: touches
                             bw                = __funnelshift_l( ab & ~gb, bw, 1 ); // A < 0 and G2 > 0: buries
                         }
-                        };
-                        if ( G == 1 )
-                            run( UnitStride {} );
-                        else
-                            run( G );
                         // into place (bit u for test u); a decided test touches when its tw bit is set
                         uw  = __brev( uw ) >> ( 32u - uN );
                         tw  = __brev( tw ) >> ( 32u - uN );
@@ -751,9 +750,9 @@ namespace sesgb
                         bur = bur | ( ( bw & ~uw ) != 0u );
                         tw |= uw; // an undecided test may touch (the touch mask is conservative)
                         // the circle's own j is always undecided and never tested
-                        const uint32_t us = s / G;
-                        if ( gl == s % G && us >= u0 && us < u0 + uN )
-                            uw &= ~( 1u << ( us - u0 ) );
+                        const uint32_t us = s - first - u0;
+                        if ( us < uN )
+                            uw &= ~( 1u << us );
                         if ( !valid )
                             uw = 0;
                         if ( u0 < 64 )
@@ -768,7 +767,7 @@ namespace sesgb
                             uint32_t at = nq + warp_exclusive_sum( (uint32_t)__popc( uw ), tot );
                             for ( uint32_t w = uw; w; w &= w - 1 )
                             {
-                                const uint32_t k = gl + G * ( u0 + (uint32_t)( __ffs( w ) - 1 ) );
+                                const uint32_t k = first + u0 + (uint32_t)( __ffs( w ) - 1 );
                                 if ( at < (uint32_t)kVisQueue )
                                     m.queue[ at ] = s | ( k << 16 );
                                 else
@@ -781,25 +780,27 @@ namespace sesgb
                 }
                 const bool gb = ( __ballot_sync( 0xffffffffu, bur ) & gmask ) != 0;
                 const bool gt = ( __ballot_sync( 0xffffffffu, tch ) & gmask ) != 0;
-                if ( ni <= (uint32_t)kMaskSlots )
+                if ( ni <= (uint32_t)kWideSlots )
                 {
-                    // touch mask of the circle over slots 0..63: the atoms that may hold
+                    // touch mask of the circle over slots 0..127: the atoms that may hold
                     // a point of it (k_probes tests only those)
-                    uint64_t x = 0;
-                    if ( G == 1 )
-                        x = (uint64_t)tou[ 0 ] | ( (uint64_t)tou[ 1 ] << 32 );
-                    else
-                        for ( uint32_t w = tou[ 0 ]; w; w &= w - 1 )
-                            x |= 1ull << ( gl + G * (uint32_t)( __ffs( w ) - 1 ) );
+                    const uint64_t t = (uint64_t)tou[ 0 ] | ( (uint64_t)tou[ 1 ] << 32 );
+                    uint64_t       x = first < 64u ? t << first : 0ull;
                     for ( uint32_t o = 1; o < G; o <<= 1 )
                         x |= __shfl_xor_sync( 0xffffffffu, x, o );
-                    if ( valid && gl == 0 && ( m.res[ s ] & kVisUpper ) )
+                    const bool     own = valid && gl == 0 && ( m.res[ s ] & kVisUpper );
+                    const uint32_t at  = own ? b.pairOff[ i ] + s : 0u;
+                    if ( own && at < b.capPairs )
+                        b.touch[ at ] = x;
+                    else if ( own )
+                        atomicOr( &b.counts->overflow, (uint32_t)kOverflowPairs );
+                    if ( ni > (uint32_t)kMaskSlots )
                     {
-                        const uint32_t at = b.pairOff[ i ] + s;
-                        if ( at < b.capPairs )
-                            b.touch[ at ] = x;
-                        else
-                            atomicOr( &b.counts->overflow, (uint32_t)kOverflowPairs );
+                        x = first == 0u || first >= 128u ? 0ull : first < 64u ? t >> ( 64u - first ) : t << ( first - 64u );
+                        for ( uint32_t o = 1; o < G; o <<= 1 )
+                            x |= __shfl_xor_sync( 0xffffffffu, x, o );
+                        if ( own && at < b.capPairs )
+                            b.touchHigh[ at ] = x;
                     }
                 }
                 if ( valid && gl == 0 && ( gb || gt ) )
@@ -815,7 +816,7 @@ namespace sesgb
                     for ( uint32_t h = 0; h < 2; h++ )
                         for ( uint32_t w = und[ h ]; w; w &= w - 1 )
                         {
-                            const uint32_t k = gl + G * ( 32 * h + (uint32_t)( __ffs( w ) - 1 ) );
+                            const uint32_t k = first + 32 * h + (uint32_t)( __ffs( w ) - 1 );
                             if ( at < (uint32_t)kVisQueue )
                                 m.queue[ at ] = s | ( k << 16 );
                             else
@@ -1369,9 +1370,10 @@ namespace sesgb
         // with a conservative error band. Sets w[e]: 0 none, +-1 regular, +-2
         // singular, +-3 kept with the singular flag undecided; or band = true
         // (both entries reserved for the double-precision pass).
+        template<bool useMask>
         __device__ __forceinline__ void probe_screen( const ProbeSmem & m, const ProbeBounds & pb, float Ri, float rp,
-                                                      uint32_t ni, bool useMask, uint32_t sj, uint32_t sk, int w[ 2 ],
-                                                      bool & band )
+                                                      uint32_t ni, const Build & b, uint32_t po, bool wide,
+                                                      uint32_t sj, uint32_t sk, int w[ 2 ], bool & band )
         {
             const float4 qj = m.rel[ sj ], qk = m.rel[ sk ];
             const f3     dj = F3( qj.x, qj.y, qj.z ), dk = F3( qk.x, qk.y, qk.z );
@@ -1423,7 +1425,7 @@ namespace sesgb
                 v2 = v2 && h2 > 0.f;
                 return ( v1 || v2 ) ? 0 : 2;
             };
-            if ( useMask )
+            if constexpr ( useMask )
             {
                 // only an atom that touches both circles (i, j) and (i, k) can hold a point of both
                 // in ascending slot order, one 32-bit half of the mask at a time
@@ -1442,15 +1444,27 @@ namespace sesgb
             }
             else
             {
-                for ( uint32_t sl = 0; sl < ni; sl++ )
+                // 32 slots at a time, by the masks in global memory or all of them
+                for ( uint32_t base = 0; base < ni; base += 32u )
                 {
-                    if ( sl == sj || sl == sk )
-                        continue;
-                    const int r = occlude( sl );
-                    if ( r )
+                    uint32_t w = 0xffffffffu >> ( ni - base < 32u ? 32u - ( ni - base ) : 0u );
+                    if ( wide )
                     {
-                        band = r == 1;
-                        return;
+                        const uint64_t * t = ( base < 64u ? b.touch : b.touchHigh ) + po;
+                        w &= (uint32_t)( ( t[ sj ] & t[ sk ] ) >> ( base & 32u ) );
+                    }
+                    if ( sj - base < 32u )
+                        w &= ~( 1u << ( sj - base ) );
+                    if ( sk - base < 32u )
+                        w &= ~( 1u << ( sk - base ) );
+                    for ( ; w; w &= w - 1 )
+                    {
+                        const int r = occlude( base + (uint32_t)( __ffs( (int)w ) - 1 ) );
+                        if ( r )
+                        {
+                            band = r == 1;
+                            return;
+                        }
                     }
                 }
             }
@@ -1470,17 +1484,20 @@ namespace sesgb
         // whose far atoms are neighbours. Entries of the atom's probe list are kept
         // in order (circle (i, j), then k, then x1 before x2) and written as one
         // chunk; positions and undecided flags are completed by k_probe_jobs.
-        __device__ __forceinline__ void probes_of_atom( const Build & b, uint32_t i, unsigned char * smemWarp )
+        // useMask: at most kMaskSlots neighbours. The two kinds of atoms are two copies of the code, the longer lists'
+        // out of line: branches for both in one slowed the common kind by a tenth.
+        template<bool useMask>
+        __device__ __forceinline__ void probes_of_neighbourhood( const Build & b, uint32_t i, unsigned char * smemWarp, uint32_t ni,
+                                                                 const float4 & ai, uint32_t po, const uint32_t * jj0, const uint32_t * st0 )
         {
             const uint32_t  lane = lane_id();
             const ProbeSmem m    = probe_smem( smemWarp, b.cap );
-            const uint32_t  ni  = b.nbrCount[ i ];
-            const float4    ai  = b.atoms[ i ];
             const float     Ri  = ai.w + b.rp;
             const size_t    row = (size_t)i * b.cap;
-            const uint32_t  po  = b.pairOff[ i ];
 
-            const bool useMask = ni <= (uint32_t)kMaskSlots;
+            // atoms of 65 to 128 neighbours (a larger probe radius): their masks stay in global memory. 6,007 atoms with a
+            // 2.4 A probe: this kernel 183 -> 102 us against trying every neighbour (25 of 80 remain)
+            const bool wide    = !useMask && ni <= (uint32_t)kWideSlots && po + ni <= b.capPairs;
             uint32_t   p       = 0;
             uint64_t   partial = 0; // slots of the partial circles (i, j), i < j
             float      d2max = 0.f, bmax = 0.f;
@@ -1488,7 +1505,7 @@ namespace sesgb
             // capacity without waiting for the count (slots past it are not used), so that they
             // travel with the atom's own loads; the neighbours' atoms, counts and touch masks
             // follow together: two round trips to memory for an atom of up to 64 neighbours
-            for ( uint32_t base0 = 0; base0 == 0 || base0 < ni; base0 += 64 )
+            for ( uint32_t base0 = 0; base0 == 0 || ( !useMask && base0 < ni ); base0 += 64 )
             {
                 uint32_t jj[ 2 ] = { 0u, 0u }, st[ 2 ] = { 0u, 0u }, cn[ 2 ] = { 0u, 0u };
                 float4   aa[ 2 ];
@@ -1497,7 +1514,12 @@ namespace sesgb
                 for ( int h = 0; h < 2; h++ )
                 {
                     const uint32_t s = base0 + 32 * h + lane;
-                    if ( s < b.cap )
+                    if ( useMask )
+                    {
+                        jj[ h ] = jj0[ h ];
+                        st[ h ] = st0[ h ];
+                    }
+                    else if ( s < b.cap )
                     {
                         jj[ h ] = b.nbr[ row + s ];
                         st[ h ] = b.status[ row + s ];
@@ -1573,7 +1595,7 @@ namespace sesgb
                     if ( lane < batch )
                     {
                         sjk = m.cand[ lane ];
-                        probe_screen( m, pb, Ri, b.rp, ni, useMask, sjk & 0xffffu, sjk >> 16, w, band );
+                        probe_screen<useMask>( m, pb, Ri, b.rp, ni, b, po, wide, sjk & 0xffffu, sjk >> 16, w, band );
                     }
                     const uint32_t need = band ? 2u : ( w[ 0 ] != 0 ) + ( w[ 1 ] != 0 );
                     uint32_t       tot;
@@ -1617,7 +1639,7 @@ namespace sesgb
                 cands += __popc( mc );
                 __syncwarp();
             };
-            if ( useMask )
+            if constexpr ( useMask )
             {
                 // for each partial circle (i, j): the partial circles (i, k), k > j, whose
                 // far atom touches circle (i, j); flattened over the circles in (j, k)
@@ -1702,6 +1724,13 @@ namespace sesgb
                             sj                = m.plist[ a ];
                             sk                = m.plist[ bb ];
                             isC               = pair_is_neighbor( b, m, pb, sj, sk, fp64 );
+                        }
+                        if ( wide )
+                        {
+                            // the far atom has to touch circle (i, j)
+                            const bool far = isC && !( ( ( sk < 64u ? b.touch : b.touchHigh )[ po + sj ] >> ( sk & 63u ) ) & 1u );
+                            cands += __popc( __ballot_sync( 0xffffffffu, far ) );
+                            isC = isC && !far;
                         }
                         enqueue( isC, sj, sk );
                     }
@@ -1868,6 +1897,35 @@ namespace sesgb
                 b.singCnt[ i ]    = fits ? nSing : 0u;
                 b.regCnt[ i ]     = fits ? nReg : 0u;
             }
+        }
+
+        __device__ __noinline__ void probes_of_long_list( const Build & b, uint32_t i, unsigned char * smemWarp )
+        {
+            const float4 ai = b.atoms[ i ];
+            probes_of_neighbourhood<false>( b, i, smemWarp, b.nbrCount[ i ], ai, b.pairOff[ i ], nullptr, nullptr );
+        }
+        __device__ __forceinline__ void probes_of_atom( const Build & b, uint32_t i, unsigned char * smemWarp )
+        {
+            // the rows travel with the atom's own loads: the branch on the count must not hold them up (without the
+            // fence it did, for 20 of 242 us at 100,000 atoms)
+            const uint32_t ni = b.nbrCount[ i ], po = b.pairOff[ i ], lane = lane_id();
+            const float4   ai = b.atoms[ i ];
+            uint32_t       jj[ 2 ] = { 0u, 0u }, st[ 2 ] = { 0u, 0u };
+#pragma unroll
+            for ( int h = 0; h < 2; h++ )
+            {
+                const uint32_t s = 32 * h + lane;
+                if ( s < b.cap )
+                {
+                    jj[ h ] = b.nbr[ (size_t)i * b.cap + s ];
+                    st[ h ] = b.status[ (size_t)i * b.cap + s ];
+                }
+            }
+            asm volatile( "" ::: "memory" );
+            if ( ni <= (uint32_t)kMaskSlots )
+                probes_of_neighbourhood<true>( b, i, smemWarp, ni, ai, po, jj, st );
+            else
+                probes_of_long_list( b, i, smemWarp );
         }
 
         // W warps per block; with kQueue the grid is persistent and its warps take tiles of atoms
