@@ -582,7 +582,7 @@ namespace sesgb
 
         // Warp per atom: convex patch and the tori of its circles (i, j), i < j. Latency- and issue-bound (12 of
         // 32 lanes, 26,000 warp instructions an atom); with the cuts of a lane's own circle in local memory and
-        // every circle walked it was 3.44 ms for 20,000 atoms (4.84 with the adjoint) and is 0.98 (1.54).
+        // every circle walked it was 3.44 ms for 20,000 atoms (4.84 with the adjoint) and is 0.75 (1.28).
         // parts (double[3]) accumulate convex, toroidal (and concave in k_area_probes);
         // atomArea (input order) receives convex + half of each torus. With kGrad,
         // gradSorted (float4 per sorted atom) accumulates gConvex d convex + gTorus d tori.
@@ -1174,8 +1174,8 @@ namespace sesgb
         }
 
         // Warp per singular probe: its concave triangle outside the listed neighbour probes. 29,500 probes of a
-        // 20,000-atom globule, the plain triangles (a thread each, 7 us) included: 0.80 ms before, 0.36 now; adjoint
-        // 3.51 and 1.0, most of it the double-precision regions.
+        // 20,000-atom globule, the plain triangles (a thread each, 7 us) included: 0.80 ms before, 0.31 now; adjoint
+        // 3.51 and 0.88, most of it the double-precision regions.
         // With kGrad, probeGrad (float4 per probe) accumulates d/d(position) of every
         // probe involved and gradSorted the direct terms of the contact directions; the lune planes
         // are not needed then.
@@ -1350,10 +1350,12 @@ namespace sesgb
             }
         }
 
+        // A warp per item: regions differ several times in their work, and 152 x 16 blocks that took every n-th item
+        // were 1.3 waves of unequal blocks (20,000 atoms: 1.01 ms, 0.75 now; with the adjoint 1.56 and 1.28)
         inline uint32_t area_blocks( uint64_t items )
         {
             const uint64_t want = ( items + kAreaWarps - 1 ) / kAreaWarps;
-            const uint64_t cap  = 152ull * 16ull;
+            const uint64_t cap  = 152ull * 8192ull;
             return (uint32_t)( want < 1 ? 1 : ( want < cap ? want : cap ) );
         }
     } // namespace
