@@ -1978,18 +1978,17 @@ namespace sesgb
         // order the host tracer writes them, so that the image does not depend on contraction
         // choices. The normal of a hit is the normalised central difference of the signed distance
         // (step normalStep) at the hit point.
-        // A warp takes 8 x 4 pixels, a lane each: their rays run close together, so that one tile
+        // A warp takes 8 x 4 pixels or fewer (rays_per_warp), a lane each: their rays run close together, so that one tile
         // search serves the warp's points; the few points it leaves go through the general search one
         // after another. Bound by the longest rays: up to maxSteps searches one after another (512 x 512
-        // pixels of a 20,000-atom globule: 28.9 ms with a warp and a general search a ray, 13.1 ms).
-        constexpr uint32_t kRaysX = 8, kRaysY = 4;
+        // pixels of a 20,000-atom globule: 28.9 ms with a warp and a general search a ray, 12.4 ms).
         __global__ void __launch_bounds__( 32 * kSdfWarps ) k_trace( Build b, SdfIndex ix, TraceParams p, float band,
-                                                                    float * depth, float * normals )
+                                                                    uint32_t logX, uint32_t logY, float * depth, float * normals )
         {
             __shared__ SdfScratch smem[ kSdfWarps ];
             const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
             uint32_t           overflow = 0;
-            const uint32_t     tilesX   = ( p.width + kRaysX - 1u ) / kRaysX, tiles = tilesX * ( ( p.height + kRaysY - 1u ) / kRaysY );
+            const uint32_t     tilesX   = ( ( p.width - 1u ) >> logX ) + 1u, tiles = tilesX * ( ( ( p.height - 1u ) >> logY ) + 1u );
             const bool         tiled    = !ix.general && ix.flags[ 2 ] == 0u;
             const float3       f        = make_float3( (float)p.forward[ 0 ], (float)p.forward[ 1 ], (float)p.forward[ 2 ] );
             const float3       r        = make_float3( (float)p.right[ 0 ], (float)p.right[ 1 ], (float)p.right[ 2 ] );
@@ -2000,8 +1999,8 @@ namespace sesgb
             const float        minStep  = __fmul_rn( 0.25f, eps );
             for ( uint32_t tile = blockIdx.x * kSdfWarps + warp; tile < tiles; tile += gridDim.x * kSdfWarps )
             {
-                const uint32_t px = ( tile % tilesX ) * kRaysX + lane % kRaysX, py = ( tile / tilesX ) * kRaysY + lane / kRaysX;
-                const bool     mine = lane < kRaysX * kRaysY && px < p.width && py < p.height;
+                const uint32_t px = ( ( tile % tilesX ) << logX ) + ( lane & ( ( 1u << logX ) - 1u ) ), py = ( ( tile / tilesX ) << logY ) + ( lane >> logX );
+                const bool     mine = lane < 1u << ( logX + logY ) && px < p.width && py < p.height;
                 // pinhole ray through the pixel centre, row-major from the top left
                 const float xs  = __fdiv_rn( __fmul_rn( __fmul_rn( __fsub_rn( __fdiv_rn( __fmul_rn( 2.f, __fadd_rn( (float)px, 0.5f ) ), W ), 1.f ),
                                                                   th ),
@@ -2264,6 +2263,17 @@ namespace sesgb
         // the arcs' bins in quarters: worth their pass from about four queries per atom on (20,000 atoms: 60,000 queries 522 us
         // without and 528 with them, 200,000 queries 913 and 850)
         bool quarters_pay( uint32_t m, uint32_t n ) { return m >= 4u * (uint64_t)n; }
+        // Pixels of a warp. A warp's time is that of its longest ray, up to maxSteps searches one after another, each
+        // of which takes 76k cycles for 8 x 4 rays and 23k for 2 x 2; in all 2 x 2 take more work. 20,000 atoms, 512 x 512 pixels:
+        // 12.9 ms with 8 x 4, 13.0 with 8 x 2, 14.0 with 4 x 2, 18.1 with 2 x 2; 384 x 384: 11.7, 8.9, 9.4, 11.2;
+        // 256 x 256: 11.5, 8.1, 7.0, 6.7 (2,000 atoms: 7.4, 5.6, 5.8, 5.8); 128 x 128: 10.4, 5.9, 4.2, 3.5
+        // (one ray 4.0); 64 x 64: 11.1, 5.5, 4.0, 3.2 (3.0).
+        void rays_per_warp( uint64_t pixels, uint32_t & logX, uint32_t & logY )
+        {
+            logX = pixels >= 3u << 15 ? 3u : pixels >= 3u << 14 ? 2u : pixels >= 3u << 11 ? 1u : 0u;
+            logY = pixels >= 3u << 16 ? 2u : pixels >= 3u << 11 ? 1u : 0u;
+        }
+
         // The general search alone, without arcs and tiles: one or a few queries, and few for the size of a large
         // molecule, whose arcs cost 5.8 us per 1000 atoms whether or not a query comes near them. Queries near the
         // surface, by the general search and by tiles: 100,000 atoms, 1000 queries 551 and 666 us, 20,000 queries 1850
@@ -2312,12 +2322,14 @@ namespace sesgb
     void launch_trace( const Build & b, const SdfState & st, const TraceParams & p, float band, float * depth, float * normals,
                        void * scratch, cudaStream_t s )
     {
-        const uint64_t tiles = (uint64_t)( ( p.width + kRaysX - 1u ) / kRaysX ) * ( ( p.height + kRaysY - 1u ) / kRaysY );
-        if ( !tiles )
+        if ( !p.width || !p.height )
             return;
+        uint32_t logX, logY;
+        rays_per_warp( (uint64_t)p.width * p.height, logX, logY );
+        const uint64_t tiles = (uint64_t)( ( ( p.width - 1u ) >> logX ) + 1u ) * ( ( ( p.height - 1u ) >> logY ) + 1u );
         uint32_t *     list, *flags;
         const SdfIndex ix = build_index( b, st, nullptr, 0, true, (uint64_t)p.width * p.height >= b.n, band, scratch, list, flags, s );
-        k_trace<<<(uint32_t)std::min<uint64_t>( blocks_of( tiles, kSdfWarps ), 152u * 64u ), 32 * kSdfWarps, 0, s>>>( b, ix, p, band, depth,
+        k_trace<<<(uint32_t)std::min<uint64_t>( blocks_of( tiles, kSdfWarps ), 152u * 64u ), 32 * kSdfWarps, 0, s>>>( b, ix, p, band, logX, logY, depth,
                                                                                                                      normals );
         count_launches( 1 );
     }

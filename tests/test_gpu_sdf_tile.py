@@ -120,3 +120,27 @@ def test_few_queries_alone_as_among_many(n, few):
     assert torch.equal(out[few], out[many][:few]) and torch.equal(kind[few], kind[many][:few])
     # one query adds to a row once; a row sums at most `few` terms of size at most 1
     assert torch.allclose(grad[few], grad[many], rtol=0, atol=few * 2.0 ** -22)
+
+
+@pytest.mark.parametrize("width,height", [(1, 1), (61, 100), (62, 100), (245, 200), (246, 200), (328, 299), (328, 300), (447, 439),
+                                          (447, 441)])
+def test_image_by_rays_per_warp(width, height):
+    # the number of pixels of a warp changes between these sizes; the general search takes a ray's points one by one
+    import torch
+    atoms = np.concatenate([synth.globule(300, 33), FAR])
+    lo, hi = atoms[:-1, :3].min(0), atoms[:-1, :3].max(0)
+    centre, rad = 0.5 * (lo + hi).astype(np.float64), 0.5 * float(np.linalg.norm(hi - lo)) + 4.0
+    cam = {"eye": centre + [0, -3.0 * rad, 0], "forward": [0, 1, 0], "right": [1, 0, 0], "up": [0, 0, 1], "tan_half_fov": 0.36,
+           "t_near": rad, "t_far": 5.0 * rad, "eps": 1e-3, "normal_step": 1e-2, "width": width, "height": height, "max_steps": 128}
+    images = []
+    for box in (None, aabb(atoms[:-1])):
+        with SesBuild(atoms, 1.4, "full", box=box) as g:
+            g.build()
+            depth = torch.full((height, width), -1.0, device="cuda")
+            normals = torch.full((height, width, 3), -1.0, device="cuda")
+            g.render(cam, depth.data_ptr(), normals.data_ptr(), torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            images.append((depth.cpu().numpy(), normals.cpu().numpy()))
+    assert width == 1 or np.isfinite(images[0][0]).any()
+    assert np.array_equal(images[0][0], images[1][0])
+    assert np.array_equal(images[0][1], images[1][1], equal_nan=True)
