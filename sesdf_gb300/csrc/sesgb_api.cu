@@ -367,7 +367,6 @@ namespace
             const ScanJob jobs[] = { { b.singCnt, b.singOff, &d->Q }, { b.regCnt, b.regOff, &d->regTotal } };
             exclusive_scan_many( jobs, 2, n, nullptr, sc, s );
         }
-        launch_zero2( b.ccount, b.ccursor, b.capC1, &d->C1, s ); // per-circle probe counts and list cursors
         launch_place( b, s );
         mark( 7 );
         const cudaStream_t sp = side ? side : s; // the stream of the probes' neighbours
@@ -380,10 +379,11 @@ namespace
         // F: segments
         if ( c->mode == SESGB_MODE_FULL )
         {
-            exclusive_scan( b.ccount, b.cstart, b.capC1, &d->C1, nullptr, sc, s );
-            launch_lists( b, s );
+            // (both scans of the circles together: two launches fewer than one before the lists and one after)
             launch_segment_counts( b, s );
-            exclusive_scan( b.segCnt, b.segOff, b.capC1, &d->C1, &d->S, sc, s );
+            const ScanJob jobs[] = { { b.ccount, b.cstart, nullptr }, { b.segCnt, b.segOff, &d->S } };
+            exclusive_scan_many( jobs, 2, b.capC1, &d->C1, sc, s );
+            launch_lists( b, s );
             launch_segments( b, s );
         }
 

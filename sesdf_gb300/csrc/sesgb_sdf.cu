@@ -1981,7 +1981,7 @@ namespace sesgb
         // A warp takes 8 x 4 pixels or fewer (rays_per_warp), a lane each: their rays run close together, so that one tile
         // search serves the warp's points; the few points it leaves go through the general search one
         // after another. Bound by the longest rays: up to maxSteps searches one after another (512 x 512
-        // pixels of a 20,000-atom globule: 28.9 ms with a warp and a general search a ray, 12.4 ms).
+        // pixels of a 20,000-atom globule: 28.9 ms with a warp and a general search a ray, 13.2 ms).
         __global__ void __launch_bounds__( 32 * kSdfWarps ) k_trace( Build b, SdfIndex ix, TraceParams p, float band,
                                                                     uint32_t logX, uint32_t logY, float * depth, float * normals )
         {

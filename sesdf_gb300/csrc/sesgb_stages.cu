@@ -998,6 +998,12 @@ namespace sesgb
         __global__ void __launch_bounds__( 32 * kWarpsPerBlock ) k_emit( Build b )
         {
             pdl_begin();
+            // zeroes the partial circles' probe counts and list cursors for k_place and k_lists (a launch of 5 us for 100,000 atoms)
+            for ( uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, C1 = min( b.counts->C1, b.capC1 ); q <= C1; q += gridDim.x * blockDim.x )
+            {
+                b.ccount[ q ]  = 0u;
+                b.ccursor[ q ] = 0u;
+            }
             const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
             const uint32_t grp = lane / kEmitGroup, gl = lane % kEmitGroup;
             const uint32_t gmask = ( ( 1u << kEmitGroup ) - 1u ) << ( grp * kEmitGroup );
