@@ -525,12 +525,12 @@ def run_ours(args, rank, world, local):
         extra["sdf_20k_1m"] = sdf_extra(flush)
         sx = extra["sdf_20k_1m"]
         # issue-rate rooflines of the on-demand kernels (their ncu summaries: profiles/<kernel>_<workload>.txt);
-        # the SDF call's time is k_sdf's to within its sort of the query keys, the area call's is the sum of
-        # k_area_atoms and k_area_probes (split by the launch list's shares)
+        # the SDF call's time is k_sdf_tile's plus its index of the arcs and the query order (a fifth), the area call's
+        # is the sum of k_area_atoms and k_area_probes (split by their shares)
         n20, m = sx["atoms"], sx["queries"]
         extra["rooflines"] = {
-            "k_sdf": issue_roofline("k_sdf", sx["forward_ms"], clocks.get("sm_mhz"), 16.0 * m + 16.0 * n20,
-                                    "globule20k_1m"),
+            "k_sdf_tile": issue_roofline("k_sdf_tile", sx["forward_ms"], clocks.get("sm_mhz"), 16.0 * m + 16.0 * n20,
+                                         "globule20k_1m"),
         }
         # the image: 16 bytes (depth + normal) per pixel out; the build it traces is L2-resident
         extra["rooflines"]["k_trace"] = issue_roofline("k_trace", sx["render_512x512_ms"], clocks.get("sm_mhz"),
@@ -581,12 +581,11 @@ REF_D2H_BYTES_EXTERIOR = 4 + 5 * 8
 
 def run_profile_case(args):
     """One on-demand workload of the 20,000-atom globule, args.steps times after args.warmup, for
-    profiler runs (no JSON line): sdf (forward and adjoint at 200,000 of the 1M queries), area
+    profiler runs (no JSON line): sdf (forward and adjoint at the 1M queries), area
     (SES area and its adjoint), render (512 x 512 depth and normal image, as timed), cavities (0.5 A voxels)."""
     import torch
     from sesdf_gb300 import SesBuild, render, synth
     atoms, q = synth.sdf_workload()
-    q = np.ascontiguousarray(q[:200_000])
     stream = torch.cuda.current_stream()
     g = SesBuild(atoms, RP, "full")
     g.build()
