@@ -597,7 +597,10 @@ namespace
             destroy_graph( c );
             c->rebuilds++;
             if ( !allocate_dynamic( c ) )
+            {
+                c->built = false; // an earlier build's buffers are gone
                 return SESGB_ERR_CUDA;
+            }
             const int st = enqueue_build( c, s, c->pendingUpload, c->pendingAtoms );
             if ( st != SESGB_OK )
                 return st;
