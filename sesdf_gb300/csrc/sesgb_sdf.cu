@@ -1877,6 +1877,14 @@ namespace sesgb
             }
         }
 
+        struct TileHit
+        {
+            SdfHit   h;
+            float3   x;
+            uint32_t query;
+        };
+        static_assert( 32 * sizeof( TileHit ) <= sizeof( TileSmem ), "a warp's hits in its tile's memory" );
+
         // Queries in cell order, G lanes each (32 / G to a warp's tile); a query left to the general
         // search goes to the list (one in 100,000). Issue- and latency-bound: 29,000 warp instructions a
         // tile of 32 at 20 of 32 lanes, where the general search took 33,000 a query at 15. 1M queries around a
@@ -1890,7 +1898,9 @@ namespace sesgb
             __shared__ TileSmem smem[ kSdfWarps ];
             const uint32_t      warp = threadIdx.x >> 5, lane = lane_id();
             const uint32_t      at   = ( blockIdx.x * kSdfWarps + warp ) * ( 32u / G ) + lane / G;
-            if ( ( blockIdx.x * kSdfWarps + warp ) * ( 32u / G ) >= m )
+            // (the adjoint's warps meet at the end)
+            const bool any = ( blockIdx.x * kSdfWarps + warp ) * ( 32u / G ) < m;
+            if ( !kBackward && !any )
                 return;
             const bool     want = at < m;
             uint32_t       qi   = 0;
@@ -1902,7 +1912,7 @@ namespace sesgb
             }
             SdfHit h;
             bool   exact = want;
-            if ( !ix.general && ix.flags[ 2 ] == 0u )
+            if ( any && !ix.general && ix.flags[ 2 ] == 0u )
                 sdf_tile_search( b, ix, x, want, G, smem[ warp ], band, h, exact );
             const bool     first = want && ( lane & ( G - 1u ) ) == 0u;
             const uint32_t mk    = __ballot_sync( 0xffffffffu, first && exact );
@@ -1910,13 +1920,37 @@ namespace sesgb
             if ( lane == 0 && mk )
                 base = atomicAdd( listCount, (uint32_t)__popc( mk ) );
             base = __shfl_sync( 0xffffffffu, base, 0 );
-            if ( !first )
-                return;
-            if ( exact )
+            if ( first && exact )
                 list[ base + __popc( mk & lanemask_lt() ) ] = qi;
-            else if ( kBackward )
-                sdf_gradient( b, h, x, gradSdf[ qi ], gradSorted );
-            else
+            if constexpr ( kBackward )
+            {
+                // The gradients of the block's queries by as few warps as hold them: a query's terms are ~150 FP64
+                // instructions of 64 cycles whatever the lanes hold (200,000 queries at G = 4: 1079 us with 8 lanes of
+                // every warp, 935 now). Few queries, whose latency is the time, don't wait for one another (500 atoms, 1000
+                // queries: 104 us, 107 with the block's wait).
+                bool         mine = first && !exact;
+                TileHit      t;
+                t.h     = h;
+                t.x     = x;
+                t.query = qi;
+                if ( G <= 8u )
+                {
+                    __syncwarp();
+                    if ( !mine )
+                        t.query = 0xffffffffu;
+                    if ( ( lane & ( G - 1u ) ) == 0u )
+                        reinterpret_cast<TileHit *>( &smem[ warp ] )[ lane / G ] = t;
+                    __syncthreads();
+                    const uint32_t each = 32u / G;
+                    mine                = threadIdx.x < kSdfWarps * each;
+                    if ( mine )
+                        t = reinterpret_cast<const TileHit *>( &smem[ threadIdx.x / each ] )[ threadIdx.x % each ];
+                    mine = mine && t.query != 0xffffffffu;
+                }
+                if ( mine )
+                    sdf_gradient( b, t.h, t.x, gradSdf[ t.query ], gradSorted );
+            }
+            else if ( first && !exact )
             {
                 sdf[ qi ] = h.value;
                 if ( kind )
