@@ -99,6 +99,7 @@ namespace
         if ( e == cudaSuccess )
             return true;
         c->err = std::string( what ) + ": " + cudaGetErrorString( e );
+        cudaGetLastError(); // reported here: the next call's launches are not to find it
         return false;
     }
 
@@ -469,6 +470,9 @@ namespace
     // enqueues one build (upload, kernels, counter read-back) without waiting
     int enqueue_build( sesgb_ctx * c, cudaStream_t s, bool upload, const void * deviceAtoms )
     {
+        // an earlier build's regrown buffers did not fit the memory of that time
+        if ( !c->dynMem && !allocate_dynamic( c ) )
+            return SESGB_ERR_CUDA;
         if ( upload && c->n )
         {
             if ( !c->hostAtoms )
@@ -564,6 +568,8 @@ namespace
     // waits for the enqueued build; on a capacity overflow regrows and builds again
     int finish_build( sesgb_ctx * c )
     {
+        if ( !c->dynMem )
+            return SESGB_ERR_NOT_BUILT; // the last build failed for want of memory: nothing is in flight
         cudaStream_t s = c->pendingStream;
         for ( int attempt = 0; attempt < 6; attempt++ )
         {
@@ -598,7 +604,7 @@ namespace
             c->rebuilds++;
             if ( !allocate_dynamic( c ) )
             {
-                c->built = false; // an earlier build's buffers are gone
+                c->built = false; // an earlier build's buffers are gone; the next build asks for new ones
                 return SESGB_ERR_CUDA;
             }
             const int st = enqueue_build( c, s, c->pendingUpload, c->pendingAtoms );
