@@ -1114,8 +1114,9 @@ extern "C"
         if ( need > c->cavBytes )
         {
             cudaFree( c->cavMem );
-            c->cavMem   = nullptr;
-            c->cavBytes = 0;
+            c->cavMem    = nullptr;
+            c->cavLabels = nullptr; // the last call's result went with its memory
+            c->cavBytes  = 0;
             if ( !cuda_ok( c, cudaMalloc( &c->cavMem, need ), "cudaMalloc" ) )
                 return SESGB_ERR_CUDA;
             c->cavBytes = need;

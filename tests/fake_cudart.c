@@ -5,8 +5,10 @@
 #include <stdlib.h>
 #include <string.h>
 
-static int      fail_mallocs, last_error;
-static unsigned launches, mallocs, frees, poke_word, poke_value, poke_left;
+static int          fail_mallocs, last_error;
+static unsigned     launches, mallocs, frees, poke_word, poke_value, poke_left;
+static const void * fill_from;
+static size_t       fill_bytes;
 
 void     fake_fail( int n ) { fail_mallocs = n; }
 unsigned fake_launches( void ) { return launches; }
@@ -17,6 +19,13 @@ void fake_poke( unsigned word, unsigned value, unsigned times )
     poke_word  = word;
     poke_value = value;
     poke_left  = times;
+}
+
+/* copies of exactly n bytes to the host read from p */
+void fake_fill( const void * p, unsigned n )
+{
+    fill_from  = p;
+    fill_bytes = n;
 }
 
 int cudaMalloc( void ** p, size_t n )
@@ -50,7 +59,7 @@ int cudaFreeHost( void * p )
 }
 int cudaMemcpy( void * d, const void * s, size_t n, int kind )
 {
-    memcpy( d, s, n );
+    memcpy( d, kind == 2 && fill_from && n == fill_bytes ? fill_from : s, n );
     if ( kind == 2 && n >= 100 && n < 256 && poke_left )
     {
         poke_left--;

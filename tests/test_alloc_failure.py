@@ -88,6 +88,30 @@ def query_buffers_fail(fake):
     assert fake.fake_live() == 0
 
 
-@pytest.mark.parametrize("body", ["regrow_fails", "query_buffers_fail"])
+def cavity_buffers_fail(fake):
+    import numpy as np
+    from sesdf_gb300 import SesBuild, SesgbError
+    atoms = np.random.default_rng(1).uniform(1, 10, (50, 4)).astype(np.float32)
+    box = np.array([0, 0, 0, 20, 20, 20], np.float64)
+    keys = box.view(np.uint64) | np.uint64(1 << 63)  # as the bounds' kernel leaves them
+    fake.fake_fill(ctypes.c_void_p(keys.ctypes.data), 48)
+    g = SesBuild(atoms, 1.4, "full")
+    g.build()
+    first = g.cavities(1.0)
+    assert len(g.cavity_labels()) == np.prod(first["dims"])
+    fake.fake_fail(1)
+    for call, error in ((lambda: g.cavities(0.25), "out of memory"), (g.cavity_labels, "not built"), (lambda: g.cavity_components(0), "not built")):
+        try:
+            call()
+            raise AssertionError("labels without memory")
+        except SesgbError as e:
+            assert error in str(e)
+    second = g.cavities(0.25)
+    assert len(g.cavity_labels()) == np.prod(second["dims"])
+    g.close()
+    assert fake.fake_live() == 0
+
+
+@pytest.mark.parametrize("body", ["regrow_fails", "query_buffers_fail", "cavity_buffers_fail"])
 def test_allocation_failure(shim, body):
     child(shim, body)
