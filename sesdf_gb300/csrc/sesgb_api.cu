@@ -964,7 +964,8 @@ extern "C"
             return SESGB_ERR_MODE;
         }
         st.rmax           = c->hCounts->rmax;
-        st.general        = c->hCounts->nbrTruncated > 0 || c->hCounts->outside > 0;
+        st.truncated      = c->hCounts->nbrTruncated > 0;
+        st.outside        = c->hCounts->outside > 0;
         const size_t need = sdf_scratch_bytes( c->b, st, m );
         if ( need > c->sdfScratchBytes )
         {

@@ -36,12 +36,15 @@ namespace sesgb
     namespace
     {
         // Cells of half the reach of a query (rmax + 2 rp + band) with, in this order in one
-        // array: the atoms, the probes, the arcs (cells each) and the queries (sub sub-cells a cell).
+        // array: the atoms, the probes, the arcs (cells each) and the queries (sub sub-cells a cell);
+        // for the general search alone the atoms and the queries.
         struct SdfIndex
         {
             FineGrid         grid;
             uint32_t         sub;     // sub-cells of a cell that order the queries: 8 (octants) or 1
-            uint32_t         general; // atoms outside the grid's box: whole stencil rows, general search only
+            uint32_t         items;   // kinds of items before the queries: 3, or 1 (atoms)
+            uint32_t         outside; // atoms outside the grid's box: whole stencil rows
+            uint32_t         tiles;   // no atoms outside, no truncated neighbour lists
             float            rmax;
             const uint32_t * start;   // (3 + sub) cells + 1
             const float4 *   pos;     // atom (x, y, z, r; r < 0 without accessible surface), probe (x, y, z, 0), arc ball (centre, radius)
@@ -222,18 +225,22 @@ namespace sesgb
         }
 
         // The general search: one query, the whole warp; the hit is valid in every lane. A point of dE
-        // within the float32 error of another SAS sphere is decided in double precision.
-        __device__ __noinline__ SdfHit sdf_query( const Build & b, const SdfIndex & ix, float3 x, SdfSmem & sm, float band,
-                                                  uint32_t & overflow )
+        // within the float32 error of another SAS sphere is decided in double precision with kExact;
+        // without, the query is only marked (exact set, in every lane) and its hit means nothing.
+        template<bool kExact>
+        __device__ __forceinline__ SdfHit sdf_query_pass( const Build & b, const SdfIndex & ix, float3 x, SdfSmem & sm, float band,
+                                                          uint32_t & overflow, bool & exact )
         {
-            const uint32_t lane = lane_id();
+            const uint32_t lane      = lane_id();
+            bool           exactLane = false;
+            exact                    = false;
             // 4 x (largest coordinate of any point of dE this query examines)
             const float qQ = 4.f * ( fmaxf( fabsf( x.x ), fmaxf( fabsf( x.y ), fabsf( x.z ) ) ) + 12.f );
             const float    T    = b.rp + band;
             // the atoms of the 5 x 5 x 5 cells around x, rows cut to the reach (whole rows where atoms lie
             // outside the grid's box and sit in its border cells)
             const uint32_t total = stencil_rows_span2( ix.grid, ix.start, make_float4( x.x, x.y, x.z, 0.f ),
-                                                       ix.general ? 3e18f : ix.rmax + b.rp + T + 0.01f, sm.rowStart, sm.rowPre );
+                                                       ix.outside ? 3e18f : ix.rmax + b.rp + T + 0.01f, sm.rowStart, sm.rowPre );
             // atoms within reach; minima of |x - c| - R (SAS) and |x - c| - r (vdW)
             uint32_t nl = 0;
             float    smin = 3.4e38f, vmin = 3.4e38f;
@@ -442,7 +449,12 @@ namespace sesgb
                         // a neighbour's sphere passes within the float32 error of the point: the point
                         // and the test in double precision
                         if ( !hid && __any_sync( 0xffffffffu, unsure ) )
-                            hid = __any_sync( 0xffffffffu, sphere_point_hidden_d( b, sm, row, nn, i, x, lane ) );
+                        {
+                            if constexpr ( kExact )
+                                hid = __any_sync( 0xffffffffu, sphere_point_hidden_d( b, sm, row, nn, i, x, lane ) );
+                            else
+                                exactLane = true;
+                        }
                         if ( !hid && lane == 0 )
                         {
                             cand = dl;
@@ -488,7 +500,12 @@ namespace sesgb
                             unsure          = unsure || !( fabsf( m ) > eb );
                         }
                         if ( !hidden && unsure )
-                            hidden = circle_point_hidden_d( b, sm, row, nn, i, s, x );
+                        {
+                            if constexpr ( kExact )
+                                hidden = circle_point_hidden_d( b, sm, row, nn, i, s, x );
+                            else
+                                exactLane = true;
+                        }
                         if ( hidden )
                             continue;
                     }
@@ -521,7 +538,23 @@ namespace sesgb
                 __syncwarp();
             }
             hit.value = b.rp - best;
+            exact     = __any_sync( 0xffffffffu, exactLane );
             return hit;
+        }
+        __device__ __noinline__ SdfHit sdf_query_exact( const Build & b, const SdfIndex & ix, float3 x, SdfSmem & sm, float band,
+                                                        uint32_t & overflow )
+        {
+            bool marked;
+            return sdf_query_pass<true>( b, ix, x, sm, band, overflow, marked );
+        }
+        // The float32 pass. Its whole hit is kept alive: without the parts that a caller does not read, the compiler arranges
+        // the loops over the neighbours so that one query took 3.1 ms instead of 2.1 (20,000 atoms, 2.9 A probe).
+        __device__ __forceinline__ SdfHit sdf_query_float( const Build & b, const SdfIndex & ix, float3 x, SdfSmem & sm, float band,
+                                                           uint32_t & overflow, bool & exact )
+        {
+            const SdfHit h = sdf_query_pass<false>( b, ix, x, sm, band, overflow, exact );
+            asm volatile( "" ::"r"( h.a ), "r"( h.b ), "r"( h.c ), "f"( h.q.x ), "f"( h.q.y ), "f"( h.q.z ) );
+            return h;
         }
 
         __device__ __forceinline__ void add_grad( float * g, uint32_t atom, float gx, float gy, float gz, float gr )
@@ -931,7 +964,7 @@ namespace sesgb
         template<bool kPlace>
         __global__ void __launch_bounds__( 256 ) k_sdf_bin( Build b, SdfIndex ix, SdfItems it )
         {
-            const uint32_t I = min( b.counts->I, b.capProbes ), A = min( ix.flags[ 0 ], it.capArcs );
+            const uint32_t I = ix.items == 3u ? min( b.counts->I, b.capProbes ) : 0u, A = min( ix.flags[ 0 ], it.capArcs );
             const uint32_t n0 = b.n, n1 = n0 + I, n2 = n1 + A, total = n2 + it.m;
             for ( uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x )
             {
@@ -971,18 +1004,18 @@ namespace sesgb
                 else
                 {
                     own = t - n2;
-                    seg = 3;
+                    seg = ix.items;
                     p   = make_float4( it.queries[ 3 * (size_t)own ], it.queries[ 3 * (size_t)own + 1 ], it.queries[ 3 * (size_t)own + 2 ], 0.f );
                 }
                 const int3 c   = fine_cell( ix.grid, p.x, p.y, p.z );
                 uint32_t   key = seg * ix.grid.cells + fine_key( ix.grid, c );
-                if ( seg == 3 && ix.sub == 8u )
+                if ( t >= n2 && ix.sub == 8u )
                 {
                     const FineGrid & g   = ix.grid;
                     const uint32_t   oct = ( p.x - g.origin.x >= ( (float)c.x + 0.5f ) * g.h ? 1u : 0u ) |
                                          ( p.y - g.origin.y >= ( (float)c.y + 0.5f ) * g.h ? 2u : 0u ) |
                                          ( p.z - g.origin.z >= ( (float)c.z + 0.5f ) * g.h ? 4u : 0u );
-                    key = 3u * g.cells + fine_key( g, c ) * 8u + oct;
+                    key = seg * g.cells + fine_key( g, c ) * 8u + oct;
                 }
                 if ( !kPlace )
                     it.rank[ t ] = atomicAdd( &it.count[ key ], 1u );
@@ -990,7 +1023,7 @@ namespace sesgb
                 {
                     const uint32_t at = ix.start[ key ] + it.rank[ t ];
                     it.id[ at ]       = own;
-                    if ( seg < 3 )
+                    if ( t < n2 )
                         it.pos[ at ] = p;
                 }
             }
@@ -1907,12 +1940,12 @@ namespace sesgb
             float3         x    = make_float3( 0.f, 0.f, 0.f );
             if ( want )
             {
-                qi = ix.id[ ix.start[ 3u * ix.grid.cells ] + at ];
+                qi = ix.id[ ix.start[ ix.items * ix.grid.cells ] + at ];
                 x  = make_float3( queries[ 3 * (size_t)qi ], queries[ 3 * (size_t)qi + 1 ], queries[ 3 * (size_t)qi + 2 ] );
             }
             SdfHit h;
             bool   exact = want;
-            if ( any && !ix.general && ix.flags[ 2 ] == 0u )
+            if ( any && ix.tiles && ix.flags[ 2 ] == 0u )
                 sdf_tile_search( b, ix, x, want, G, smem[ warp ], band, h, exact );
             const bool     first = want && ( lane & ( G - 1u ) ) == 0u;
             const uint32_t mk    = __ballot_sync( 0xffffffffu, first && exact );
@@ -1958,22 +1991,71 @@ namespace sesgb
             }
         }
 
-        // the listed queries (without a list: all m, in cell order) by the general search, a warp each; six blocks a SM: 1M
-        // atoms, 40,000 queries 5221 us (5764 with four, 4774 with eight, whose spills cost a lone query 13 %)
+        // All m queries by the general search, a warp each, in cell order: the float32 pass; what it leaves open goes
+        // to the list. Nothing here calls a function with the build (but for a gradient), and the pass fits 64 registers: eight blocks
+        // a SM. Issue-bound (51 % at 15 of 32 lanes). 200,000 queries of 20,001 atoms one of which lies outside the box: 17.7 ms
+        // with both passes in one function at six blocks, 9.9 now; 1M atoms, 40,000 queries 3.75 and 2.9 ms.
         template<bool kBackward>
-        __global__ void __launch_bounds__( 32 * kSdfWarps, 6 ) k_sdf_exact( Build b, SdfIndex ix, const float * queries, float band, float * sdf,
-                                                                      const float * gradSdf, float * gradSorted, int * kind,
-                                                                      const uint32_t * list, const uint32_t * listCount, uint32_t m )
+        __global__ void __launch_bounds__( 32 * kSdfWarps, 8 ) k_sdf_general( const __grid_constant__ Build b, const __grid_constant__ SdfIndex ix,
+                                                                              const float * queries, uint32_t m, float band, float * sdf,
+                                                                              const float * gradSdf, float * gradSorted, int * kind, uint32_t * list,
+                                                                              uint32_t * listCount )
         {
             __shared__ SdfSmem smem[ kSdfWarps ];
             const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
-            const uint32_t     count = list ? *listCount : m;
+            uint32_t           overflow = 0;
+            for ( uint32_t e = blockIdx.x * kSdfWarps + warp; e < m; e += gridDim.x * kSdfWarps )
+            {
+                const uint32_t qi = ix.id[ ix.start[ ix.items * ix.grid.cells ] + e ];
+                const float3   x  = make_float3( queries[ 3 * (size_t)qi ], queries[ 3 * (size_t)qi + 1 ], queries[ 3 * (size_t)qi + 2 ] );
+                bool           exact;
+                const SdfHit   h = sdf_query_float( b, ix, x, smem[ warp ], band, overflow, exact );
+                if ( lane == 0 )
+                {
+                    if ( exact )
+                        list[ atomicAdd( listCount, 1u ) ] = qi;
+                    else if ( kBackward )
+                        sdf_gradient( b, h, x, gradSdf[ qi ], gradSorted );
+                    else
+                    {
+                        sdf[ qi ] = h.value;
+                        if ( kind )
+                            kind[ qi ] = h.kind;
+                    }
+                }
+                __syncwarp();
+            }
+            if ( lane == 0 && overflow )
+                atomicOr( &b.counts->overflow, (uint32_t)kOverflowSdfList );
+        }
+
+        // The listed queries by the general search in double precision where it takes that, a warp each: the few that the
+        // tile search or the float32 pass left open, whose latency counts (1M atoms, 50,000 queries: 46 us less with five blocks
+        // a SM, which need no spills, than with eight); and every query of a build that cannot take tiles, those through float32 first.
+        template<bool kBackward>
+        __global__ void __launch_bounds__( 32 * kSdfWarps, 5 ) k_sdf_exact( const __grid_constant__ Build b, const __grid_constant__ SdfIndex ix,
+                                                                            const float * queries, float band, float * sdf, const float * gradSdf,
+                                                                            float * gradSorted, int * kind, const uint32_t * list,
+                                                                            const uint32_t * listCount )
+        {
+            __shared__ SdfSmem smem[ kSdfWarps ];
+            const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
+            const uint32_t     count = *listCount;
+            const bool         all   = ix.open && ( !ix.tiles || ix.flags[ 2 ] != 0u );
             uint32_t           overflow = 0;
             for ( uint32_t e = blockIdx.x * kSdfWarps + warp; e < count; e += gridDim.x * kSdfWarps )
             {
-                const uint32_t qi = list ? list[ e ] : ix.id[ ix.start[ 3u * ix.grid.cells ] + e ];
+                const uint32_t qi = list[ e ];
                 const float3 x = make_float3( queries[ 3 * (size_t)qi ], queries[ 3 * (size_t)qi + 1 ], queries[ 3 * (size_t)qi + 2 ] );
-                const SdfHit h = sdf_query( b, ix, x, smem[ warp ], band, overflow );
+                SdfHit       h;
+                bool         exact = true;
+                if ( all )
+                {
+                    h = sdf_query_float( b, ix, x, smem[ warp ], band, overflow, exact );
+                    __syncwarp();
+                }
+                if ( exact )
+                    h = sdf_query_exact( b, ix, x, smem[ warp ], band, overflow );
                 if ( lane == 0 )
                 {
                     if ( kBackward )
@@ -2023,7 +2105,7 @@ namespace sesgb
             const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
             uint32_t           overflow = 0;
             const uint32_t     tilesX   = ( ( p.width - 1u ) >> logX ) + 1u, tiles = tilesX * ( ( ( p.height - 1u ) >> logY ) + 1u );
-            const bool         tiled    = !ix.general && ix.flags[ 2 ] == 0u;
+            const bool         tiled    = ix.tiles && ix.flags[ 2 ] == 0u;
             const float3       f        = make_float3( (float)p.forward[ 0 ], (float)p.forward[ 1 ], (float)p.forward[ 2 ] );
             const float3       r        = make_float3( (float)p.right[ 0 ], (float)p.right[ 1 ], (float)p.right[ 2 ] );
             const float3       u        = make_float3( (float)p.up[ 0 ], (float)p.up[ 1 ], (float)p.up[ 2 ] );
@@ -2108,7 +2190,7 @@ namespace sesgb
                         const float3 xs  = make_float3( __shfl_sync( 0xffffffffu, q.x, src ), __shfl_sync( 0xffffffffu, q.y, src ),
                                                         __shfl_sync( 0xffffffffu, q.z, src ) );
                         __syncwarp();
-                        const SdfHit hs = sdf_query( b, ix, xs, smem[ warp ].query, band, overflow );
+                        const SdfHit hs = sdf_query_exact( b, ix, xs, smem[ warp ].query, band, overflow );
                         __syncwarp();
                         if ( (int)lane == src )
                         {
@@ -2181,20 +2263,22 @@ namespace sesgb
         uint32_t arc_capacity( uint32_t n ) { return 16u * n + 4096u; }
 
         // Cells of half a query's reach over the reference grid's box, coarsened until they fit
-        // (a sparse molecule)
-        void index_grid( const Build & b, float rmax, float band, uint32_t m, FineGrid & g, uint32_t & sub )
+        // (a sparse molecule). For the general search alone 0.7 of it: fewer cells to zero and to scan, where few queries
+        // meet a large molecule (1,000 of 1M atoms 729 us with a half, 678 with 0.7, 716 with 1.0), and no slower
+        // elsewhere, as the rows of cells are cut to the reach; with atoms outside the box they are not.
+        void index_grid( const Build & b, const SdfState & st, float band, uint32_t m, uint32_t items, FineGrid & g, uint32_t & sub )
         {
             const double   size = b.grid.size;
             const double   e[ 3 ] = { b.grid.cell.x * size, b.grid.cell.y * size, b.grid.cell.z * size };
             const uint64_t most = std::min<uint64_t>( std::max<uint64_t>( 1u << 18, 24ull * b.n + 4ull * m ), 1u << 28 );
             sub                 = m ? 8u : 0u;
-            double h            = 0.5 * ( rmax + 2.0 * b.rp + band );
+            double h            = ( items == 1u && !st.outside ? 0.7 : 0.5 ) * ( st.rmax + 2.0 * b.rp + band );
             int    d[ 3 ]       = { 1, 1, 1 };
             for ( int it = 0; it < 400; it++ )
             {
                 for ( int a = 0; a < 3; a++ )
                     d[ a ] = b.n && e[ a ] >= 0.0 && std::isfinite( e[ a ] ) ? (int)std::min( std::max( 1.0, std::ceil( e[ a ] / h ) ), 1e6 ) : 1;
-                if ( (uint64_t)d[ 0 ] * d[ 1 ] * d[ 2 ] * ( 3u + sub ) <= most )
+                if ( (uint64_t)d[ 0 ] * d[ 1 ] * d[ 2 ] * ( items + sub ) <= most )
                     break;
                 if ( sub == 8u )
                     sub = 1u;
@@ -2212,10 +2296,11 @@ namespace sesgb
         {
             size_t flags, balls, arcs, open, count, start, rank, pos, id, list, scan, total;
         };
-        SdfLayout layout_of( const Build & b, const FineGrid & g, uint32_t sub, uint32_t m )
+        SdfLayout layout_of( const Build & b, const FineGrid & g, uint32_t sub, uint32_t kinds, uint32_t m )
         {
-            const uint64_t items = (uint64_t)b.n + b.capProbes + arc_capacity( b.n );
-            const uint64_t cells = (uint64_t)g.cells * ( 3u + sub );
+            const bool     arcs  = kinds == 3u;
+            const uint64_t items = b.n + ( arcs ? (uint64_t)b.capProbes + arc_capacity( b.n ) : 0ull );
+            const uint64_t cells = (uint64_t)g.cells * ( kinds + sub );
             SdfLayout      L;
             size_t         p = 0;
             auto           take = [ & ]( size_t bytes ) {
@@ -2226,9 +2311,9 @@ namespace sesgb
             L.flags = take( 16 );
             L.count = take( cells * 4 ); // zeroed together with the flags
             L.start = take( ( cells + 1 ) * 4 );
-            L.balls = take( (size_t)arc_capacity( b.n ) * 16 );
-            L.arcs  = take( (size_t)arc_capacity( b.n ) * 8 );
-            L.open  = take( (size_t)b.n * 32 );
+            L.balls = take( arcs ? (size_t)arc_capacity( b.n ) * 16 : 0 );
+            L.arcs  = take( arcs ? (size_t)arc_capacity( b.n ) * 8 : 0 );
+            L.open  = take( arcs ? (size_t)b.n * 32 : 0 );
             L.rank  = take( ( items + m ) * 4 );
             L.pos   = take( items * 16 );
             L.id    = take( ( items + m ) * 4 );
@@ -2244,8 +2329,9 @@ namespace sesgb
                               void * scratch, uint32_t *& list, uint32_t *& flags, cudaStream_t s )
         {
             SdfIndex ix;
-            index_grid( b, st.rmax, band, m, ix.grid, ix.sub );
-            const SdfLayout L = layout_of( b, ix.grid, ix.sub, m );
+            ix.items = arcs ? 3u : 1u;
+            index_grid( b, st, band, m, ix.items, ix.grid, ix.sub );
+            const SdfLayout L = layout_of( b, ix.grid, ix.sub, ix.items, m );
             char *          p = static_cast<char *>( scratch );
             flags             = reinterpret_cast<uint32_t *>( p + L.flags );
             list              = reinterpret_cast<uint32_t *>( p + L.list );
@@ -2259,7 +2345,8 @@ namespace sesgb
             it.pos     = reinterpret_cast<float4 *>( p + L.pos );
             it.id      = reinterpret_cast<uint32_t *>( p + L.id );
             uint32_t * start = reinterpret_cast<uint32_t *>( p + L.start );
-            ix.general = st.general ? 1u : 0u;
+            ix.outside = st.outside ? 1u : 0u;
+            ix.tiles   = st.truncated || st.outside ? 0u : 1u;
             ix.rmax    = st.rmax;
             ix.start   = start;
             ix.pos     = it.pos;
@@ -2274,7 +2361,7 @@ namespace sesgb
                                                                                   reinterpret_cast<uint32_t *>( p + L.open ), quarters, flags );
             const uint32_t blocks = (uint32_t)std::min<uint64_t>( 152u * 8u, blocks_of( 8ull * b.n + m + 1, 256 ) );
             k_sdf_bin<false><<<blocks, 256, 0, s>>>( b, ix, it );
-            exclusive_scan( it.count, start, (uint64_t)ix.grid.cells * ( 3u + ix.sub ), nullptr, nullptr, p + L.scan, s );
+            exclusive_scan( it.count, start, (uint64_t)ix.grid.cells * ( ix.items + ix.sub ), nullptr, nullptr, p + L.scan, s );
             k_sdf_bin<true><<<blocks, 256, 0, s>>>( b, ix, it );
             count_launches( arcs ? 3 : 2 );
             return ix;
@@ -2309,11 +2396,17 @@ namespace sesgb
         }
 
         // The general search alone, without arcs and tiles: one or a few queries, and few for the size of a large
-        // molecule, whose arcs cost 5.8 us per 1000 atoms whether or not a query comes near them. Queries near the
-        // surface, by the general search and by tiles: 100,000 atoms, 1000 queries 551 and 666 us, 20,000 queries 1850
-        // and 916; 300,000 atoms, 6000 queries 1076 and 1890, 20,000 queries 2526 and 2095; 20,000 atoms, 1 query 96 and 173,
-        // 4 queries 252 and 178.
-        bool general_only( uint32_t m, uint32_t n ) { return 12500ull * m <= n || 20ull * m + 52000u < n; }
+        // molecule, whose arcs cost 5.6 us per 1000 atoms whether or not a query comes near them. Queries near the
+        // surface, by the general search and by tiles: 20,000 atoms, 1 query 311 and 186 us (78 and 178 for one in the
+        // molecule's box), 2 queries 349 and 183; 100,000 atoms, 5000 queries 634 and 705, 7000 746 and 725; 300,000 atoms,
+        // 20,000 queries 1522 and 2071, 26,000 2136 and 2146; 1,000,000 atoms, 100,000 queries 5579 and 7478, 150,000 8438 and
+        // 8131. Uniform in the box the lines lie 10 to 20 % higher.
+        bool general_only( uint32_t m, uint32_t n ) { return 12500ull * m <= n || 9ull * m + 55000u < n; }
+        // m: queries, 0 for an image
+        bool general_search( const Build & b, uint32_t m )
+        {
+            return m && general_only( m, b.n );
+        }
 
         template<bool kBackward>
         void launch_search( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,
@@ -2321,19 +2414,22 @@ namespace sesgb
         {
             const uint32_t exactBlocks = std::min( blocks_of( m, kSdfWarps ), 152u * 8u );
             uint32_t *     list, *flags;
-            if ( general_only( m, b.n ) )
+            if ( general_search( b, m ) )
             {
                 const SdfIndex ix = build_index( b, st, queries, m, false, false, band, scratch, list, flags, s );
-                k_sdf_exact<kBackward><<<blocks_of( m, kSdfWarps ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, nullptr,
-                                                                              nullptr, m );
-                count_launches( 1 );
+                // (more blocks than that would each wait for the longest of its queries: 1M atoms, 100,000 queries 5838 us, 5579 with
+                // warps that go on by themselves; few of these would leave SMs without work at the end)
+                k_sdf_general<kBackward><<<std::min( blocks_of( m, kSdfWarps ), 152u * 32u ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, sdf, gradSdf, gradSorted, kind,
+                                                                                              list, flags + 1 );
+                k_sdf_exact<kBackward><<<exactBlocks, 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, list, flags + 1 );
+                count_launches( 2 );
                 return;
             }
             const SdfIndex ix = build_index( b, st, queries, m, true, quarters_pay( m, b.n ), band, scratch, list, flags, s );
             const uint32_t G  = lanes_per_query( m, b.n );
             k_sdf_tile<kBackward><<<blocks_of( (uint64_t)m * G, 32 * kSdfWarps ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, G, sdf, gradSdf,
                                                                                                           gradSorted, kind, list, flags + 1 );
-            k_sdf_exact<kBackward><<<exactBlocks, 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, list, flags + 1, m );
+            k_sdf_exact<kBackward><<<exactBlocks, 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, list, flags + 1 );
             count_launches( 2 );
         }
     } // namespace
@@ -2342,8 +2438,9 @@ namespace sesgb
     {
         FineGrid g;
         uint32_t sub;
-        index_grid( b, st.rmax, SESGB_SDF_BAND, m, g, sub );
-        return layout_of( b, g, sub, m ).total;
+        const uint32_t items = general_search( b, m ) ? 1u : 3u;
+        index_grid( b, st, SESGB_SDF_BAND, m, items, g, sub );
+        return layout_of( b, g, sub, items, m ).total;
     }
 
     void launch_sdf( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,

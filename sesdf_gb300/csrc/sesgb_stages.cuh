@@ -141,8 +141,9 @@ namespace sesgb
     // signed distance to the SES at float3 query points (sesgb_sdf.cu)
     struct SdfState
     {
-        float rmax;    // largest vdW radius of the build
-        bool  general; // truncated neighbour lists, or atoms outside the grid's box: the general search alone
+        float rmax;      // largest vdW radius of the build
+        bool  truncated; // neighbour lists
+        bool  outside;   // atoms outside the grid's box
     };
     size_t sdf_scratch_bytes( const Build & b, const SdfState & st, uint32_t m );
     void   launch_sdf( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,
