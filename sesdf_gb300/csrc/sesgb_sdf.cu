@@ -1945,7 +1945,7 @@ namespace sesgb
             }
             SdfHit h;
             bool   exact = want;
-            if ( any && ix.tiles && ix.flags[ 2 ] == 0u )
+            if ( any && ix.flags[ 2 ] == 0u )
                 sdf_tile_search( b, ix, x, want, G, smem[ warp ], band, h, exact );
             const bool     first = want && ( lane & ( G - 1u ) ) == 0u;
             const uint32_t mk    = __ballot_sync( 0xffffffffu, first && exact );
@@ -2031,7 +2031,7 @@ namespace sesgb
 
         // The listed queries by the general search in double precision where it takes that, a warp each: the few that the
         // tile search or the float32 pass left open, whose latency counts (1M atoms, 50,000 queries: 46 us less with five blocks
-        // a SM, which need no spills, than with eight); and every query of a build that cannot take tiles, those through float32 first.
+        // a SM, which need no spills, than with eight); and every query where the arcs did not fit, those through float32 first.
         template<bool kBackward>
         __global__ void __launch_bounds__( 32 * kSdfWarps, 5 ) k_sdf_exact( const __grid_constant__ Build b, const __grid_constant__ SdfIndex ix,
                                                                             const float * queries, float band, float * sdf, const float * gradSdf,
@@ -2041,7 +2041,7 @@ namespace sesgb
             __shared__ SdfSmem smem[ kSdfWarps ];
             const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
             const uint32_t     count = *listCount;
-            const bool         all   = ix.open && ( !ix.tiles || ix.flags[ 2 ] != 0u );
+            const bool         all   = ix.flags[ 2 ] != 0u;
             uint32_t           overflow = 0;
             for ( uint32_t e = blockIdx.x * kSdfWarps + warp; e < count; e += gridDim.x * kSdfWarps )
             {
@@ -2367,6 +2367,22 @@ namespace sesgb
             return ix;
         }
 
+        // Builds whose queries all take the general search: truncated neighbour lists, atoms outside the box, and
+        // SAS spheres or coordinates so large that the ball of an arc piece can pass kArcBall (k_sdf_arcs: half a piece is at most
+        // kArcHalf long, or half a bin of the largest circle).
+        bool general_build( const Build & b, const SdfState & st )
+        {
+            const float R    = st.rmax + b.rp;
+            const float half = std::max( kArcHalf + 1.1e-3f * R, R * std::sin( 0.5f * kArcStep + 1e-3f ) );
+            float       far  = 0.f;
+            for ( int a = 0; a < 3; a++ )
+            {
+                const float lo = ( &b.grid.origin.x )[ a ], hi = lo + ( &b.grid.cell.x )[ a ] * (float)b.grid.size;
+                far            = std::max( far, std::max( std::fabs( lo ), std::fabs( hi ) ) );
+            }
+            return st.truncated || st.outside || !( half + 1e-3f + 1e-6f * far < kArcBall );
+        }
+
         // Lanes per query. Few queries per atom make the tile of a warp wide, so that its lists are long, and few queries
         // leave the GPU idle; more lanes per query make the tile smaller and the walk over its lists shorter, and cost
         // the tile's own work again. Measured over 2,000 to 100,000 atoms and 1,000 to 1,000,000 queries in the molecule's
@@ -2403,9 +2419,9 @@ namespace sesgb
         // 8131. Uniform in the box the lines lie 10 to 20 % higher.
         bool general_only( uint32_t m, uint32_t n ) { return 12500ull * m <= n || 9ull * m + 55000u < n; }
         // m: queries, 0 for an image
-        bool general_search( const Build & b, uint32_t m )
+        bool general_search( const Build & b, const SdfState & st, uint32_t m )
         {
-            return m && general_only( m, b.n );
+            return m && ( general_build( b, st ) || general_only( m, b.n ) );
         }
 
         template<bool kBackward>
@@ -2414,7 +2430,7 @@ namespace sesgb
         {
             const uint32_t exactBlocks = std::min( blocks_of( m, kSdfWarps ), 152u * 8u );
             uint32_t *     list, *flags;
-            if ( general_search( b, m ) )
+            if ( general_search( b, st, m ) )
             {
                 const SdfIndex ix = build_index( b, st, queries, m, false, false, band, scratch, list, flags, s );
                 // (more blocks than that would each wait for the longest of its queries: 1M atoms, 100,000 queries 5838 us, 5579 with
@@ -2438,7 +2454,7 @@ namespace sesgb
     {
         FineGrid g;
         uint32_t sub;
-        const uint32_t items = general_search( b, m ) ? 1u : 3u;
+        const uint32_t items = general_search( b, st, m ) ? 1u : 3u;
         index_grid( b, st, SESGB_SDF_BAND, m, items, g, sub );
         return layout_of( b, g, sub, items, m ).total;
     }

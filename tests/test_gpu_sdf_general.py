@@ -1,0 +1,70 @@
+"""Builds whose signed distance takes the general search alone: truncated neighbour lists, atoms outside the box,
+spheres of tens of A; and arcs in more pieces than their buffer holds, which only the device finds out. The values are
+those of the general search on the same molecule with an atom outside its box, and nothing is launched for tiles."""
+import numpy as np
+import pytest
+
+from sesdf_gb300 import SesBuild, api, synth
+from sesdf_gb300.api import aabb
+from test_gpu_sdf_tile import evaluate
+
+pytestmark = pytest.mark.gpu
+
+
+def launches(call):
+    lib = api.load_library()
+    before = lib.sesgb_launch_count()
+    call()
+    return lib.sesgb_launch_count() - before
+
+
+def pairs(n):
+    # 64 pieces for the circle of two spheres of 15 A, more than 16 an atom
+    g = np.arange(8, dtype=np.float32) * 80.0
+    c = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)[: n // 2]
+    a = np.concatenate([np.c_[c, np.full(n // 2, 13.0)], np.c_[c + np.float32([6.0, 1.0, 2.0]), np.full(n // 2, 13.5)]])
+    return a.astype(np.float32)
+
+
+MOLECULES = {"pieces do not fit": (lambda: pairs(800), 1.4), "beads": (lambda: synth.globule(400, 61) * np.float32(13.0), 2.0)}
+
+
+@pytest.mark.parametrize("name", sorted(MOLECULES))
+def test_values_are_those_of_the_general_search(name):
+    make, rp = MOLECULES[name]
+    atoms = make()
+    far = np.float32([[*(atoms[:, :3].max(0) + 2000.0), 1.5]])
+    both = np.concatenate([atoms, far])
+    rng = np.random.default_rng(8)
+    k = rng.integers(0, len(atoms), 3000)
+    d = rng.normal(size=(3000, 3))
+    q = (atoms[k, :3] + d / np.linalg.norm(d, axis=1)[:, None] * (atoms[k, 3:] + rng.uniform(-0.9 * rp, 1.5, (3000, 1)))).astype(np.float32)
+    gq = rng.standard_normal(len(q)).astype(np.float32)
+    out = []
+    for box in (None, aabb(atoms)):
+        with SesBuild(both, rp, "full", box=box, max_neighbor_per_atom=288) as g:
+            g.build()
+            assert g.counts()["outside_atoms"] == (box is not None) and g.counts()["truncated_atoms"] == 0
+            out.append(evaluate(g, q, gq))
+    (got, kind, grad), (want, wkind, wgrad) = out
+    assert np.array_equal(got, want) and np.mean(kind == wkind) > 0.999
+    assert len(np.unique(kind)) > 3
+    assert np.linalg.norm(grad - wgrad) <= 1e-4 * np.linalg.norm(wgrad)
+
+
+def test_general_builds_launch_nothing_for_tiles():
+    # without truncated lists one kernel more, for the arcs
+    import torch
+    atoms = synth.globule(1500, 62)
+    q = torch.from_numpy(synth.queries(atoms, 1000, 3)).cuda()
+    out, grad = torch.empty(1000, device="cuda"), torch.empty(1500, 4, device="cuda")
+    counts = []
+    for slots in (16, 128):
+        with SesBuild(atoms, 1.4, "full", max_neighbor_per_atom=slots) as g:
+            g.build()
+            assert (g.counts()["truncated_atoms"] > 0) == (slots == 16)
+            counts.append([launches(lambda: g.sdf(q.data_ptr(), 1000, out.data_ptr())),
+                           launches(lambda: g.sdf_backward(q.data_ptr(), 1000, out.data_ptr(), grad.data_ptr()))])
+            torch.cuda.synchronize()
+    # (the scan of the general search's fewer cells may be a launch shorter too)
+    assert all(t - g >= less for g, t, less in zip(*counts, (1, 1)))
