@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 #include "../../include/sesgb.h"
 #include "sesgb_grid.cuh"
@@ -44,7 +45,6 @@ namespace sesgb
             uint32_t         sub;     // sub-cells of a cell that order the queries: 8 (octants) or 1
             uint32_t         items;   // kinds of items before the queries: 3, or 1 (atoms)
             uint32_t         outside; // atoms outside the grid's box: whole stencil rows
-            uint32_t         tiles;   // no atoms outside, no truncated neighbour lists
             float            rmax;
             const uint32_t * start;   // (3 + sub) cells + 1
             const float4 *   pos;     // atom (x, y, z, r; r < 0 without accessible surface), probe (x, y, z, 0), arc ball (centre, radius)
@@ -2098,14 +2098,19 @@ namespace sesgb
         // search serves the warp's points; the few points it leaves go through the general search one
         // after another. Bound by the longest rays: up to maxSteps searches one after another (512 x 512
         // pixels of a 20,000-atom globule: 28.9 ms with a warp and a general search a ray, 13.2 ms).
-        __global__ void __launch_bounds__( 32 * kSdfWarps ) k_trace( Build b, SdfIndex ix, TraceParams p, float band,
-                                                                    uint32_t logX, uint32_t logY, float * depth, float * normals )
+        // kTiles false: the general search alone, a warp per ray.
+        template<bool kTiles>
+        __global__ void __launch_bounds__( 32 * kSdfWarps, kTiles ? 4 : 6 ) k_trace( const __grid_constant__ Build b, const __grid_constant__ SdfIndex ix,
+                                                                                     const __grid_constant__ TraceParams p, float band,
+                                                                                     uint32_t logX, uint32_t logY, float * depth, float * normals )
         {
-            __shared__ SdfScratch smem[ kSdfWarps ];
+            __shared__ std::conditional_t<kTiles, SdfScratch, SdfSmem> smem[ kSdfWarps ];
             const uint32_t     warp = threadIdx.x >> 5, lane = lane_id();
             uint32_t           overflow = 0;
             const uint32_t     tilesX   = ( ( p.width - 1u ) >> logX ) + 1u, tiles = tilesX * ( ( ( p.height - 1u ) >> logY ) + 1u );
-            const bool         tiled    = ix.tiles && ix.flags[ 2 ] == 0u;
+            // with arcs both kernels are launched: where the pieces fitted, the tiles' takes the image
+            if ( ix.open && kTiles == ( ix.flags[ 2 ] != 0u ) )
+                return;
             const float3       f        = make_float3( (float)p.forward[ 0 ], (float)p.forward[ 1 ], (float)p.forward[ 2 ] );
             const float3       r        = make_float3( (float)p.right[ 0 ], (float)p.right[ 1 ], (float)p.right[ 2 ] );
             const float3       u        = make_float3( (float)p.up[ 0 ], (float)p.up[ 1 ], (float)p.up[ 2 ] );
@@ -2115,8 +2120,9 @@ namespace sesgb
             const float        minStep  = __fmul_rn( 0.25f, eps );
             for ( uint32_t tile = blockIdx.x * kSdfWarps + warp; tile < tiles; tile += gridDim.x * kSdfWarps )
             {
-                const uint32_t px = ( ( tile % tilesX ) << logX ) + ( lane & ( ( 1u << logX ) - 1u ) ), py = ( ( tile / tilesX ) << logY ) + ( lane >> logX );
-                const bool     mine = lane < 1u << ( logX + logY ) && px < p.width && py < p.height;
+                const uint32_t at0 = kTiles ? lane : 0u; // pixel of the tile (without tiles all lanes march the one ray)
+                const uint32_t px = ( ( tile % tilesX ) << logX ) + ( at0 & ( ( 1u << logX ) - 1u ) ), py = ( ( tile / tilesX ) << logY ) + ( at0 >> logX );
+                const bool     mine = at0 < 1u << ( logX + logY ) && px < p.width && py < p.height;
                 // pinhole ray through the pixel centre, row-major from the top left
                 const float xs  = __fdiv_rn( __fmul_rn( __fmul_rn( __fsub_rn( __fdiv_rn( __fmul_rn( 2.f, __fadd_rn( (float)px, 0.5f ) ), W ), 1.f ),
                                                                   th ),
@@ -2158,9 +2164,18 @@ namespace sesgb
                             q.z = __fadd_rn( xh.z, e );
                     }
                     SdfHit h;
-                    bool   exact = live;
-                    if ( tiled )
+                    if constexpr ( !kTiles )
                     {
+                        bool exact;
+                        __syncwarp();
+                        h = sdf_query_float( b, ix, q, smem[ warp ], band, overflow, exact );
+                        __syncwarp();
+                        if ( exact )
+                            h = sdf_query_exact( b, ix, q, smem[ warp ], band, overflow );
+                    }
+                    else
+                    {
+                        bool exact = live;
                         // the rays still live, side by side, with all lanes shared among them (the last rays of a
                         // tile, up to maxSteps steps long, decide when the image is done)
                         const uint32_t rays = __ballot_sync( 0xffffffffu, live ), count = (uint32_t)__popc( rays );
@@ -2183,19 +2198,19 @@ namespace sesgb
                         h.kind         = __shfl_sync( 0xffffffffu, h.kind, from );
                         h.value        = __shfl_sync( 0xffffffffu, h.value, from );
                         exact          = __shfl_sync( 0xffffffffu, ex ? 1 : 0, from ) != 0;
-                    }
-                    for ( uint32_t left = __ballot_sync( 0xffffffffu, live && exact ); left; left &= left - 1u )
-                    {
-                        const int    src = __ffs( (int)left ) - 1;
-                        const float3 xs  = make_float3( __shfl_sync( 0xffffffffu, q.x, src ), __shfl_sync( 0xffffffffu, q.y, src ),
-                                                        __shfl_sync( 0xffffffffu, q.z, src ) );
-                        __syncwarp();
-                        const SdfHit hs = sdf_query_exact( b, ix, xs, smem[ warp ].query, band, overflow );
-                        __syncwarp();
-                        if ( (int)lane == src )
+                        for ( uint32_t left = __ballot_sync( 0xffffffffu, live && exact ); left; left &= left - 1u )
                         {
-                            h.kind  = hs.kind;
-                            h.value = hs.value;
+                            const int    src = __ffs( (int)left ) - 1;
+                            const float3 xs  = make_float3( __shfl_sync( 0xffffffffu, q.x, src ), __shfl_sync( 0xffffffffu, q.y, src ),
+                                                            __shfl_sync( 0xffffffffu, q.z, src ) );
+                            __syncwarp();
+                            const SdfHit hs = sdf_query_exact( b, ix, xs, smem[ warp ].query, band, overflow );
+                            __syncwarp();
+                            if ( (int)lane == src )
+                            {
+                                h.kind  = hs.kind;
+                                h.value = hs.value;
+                            }
                         }
                     }
                     if ( !live )
@@ -2237,7 +2252,7 @@ namespace sesgb
                     const float inv = gl > 0.f ? gl : 1.f;
                     nrm = make_float3( __fdiv_rn( g.x, inv ), __fdiv_rn( g.y, inv ), __fdiv_rn( g.z, inv ) );
                 }
-                if ( mine )
+                if ( mine && ( kTiles || lane == 0u ) )
                 {
                     const size_t at = (size_t)py * p.width + px;
                     depth[ at ]     = hit;
@@ -2346,7 +2361,6 @@ namespace sesgb
             it.id      = reinterpret_cast<uint32_t *>( p + L.id );
             uint32_t * start = reinterpret_cast<uint32_t *>( p + L.start );
             ix.outside = st.outside ? 1u : 0u;
-            ix.tiles   = st.truncated || st.outside ? 0u : 1u;
             ix.rmax    = st.rmax;
             ix.start   = start;
             ix.pos     = it.pos;
@@ -2421,7 +2435,7 @@ namespace sesgb
         // m: queries, 0 for an image
         bool general_search( const Build & b, const SdfState & st, uint32_t m )
         {
-            return m && ( general_build( b, st ) || general_only( m, b.n ) );
+            return general_build( b, st ) || ( m && general_only( m, b.n ) );
         }
 
         template<bool kBackward>
@@ -2471,13 +2485,21 @@ namespace sesgb
     {
         if ( !p.width || !p.height )
             return;
-        uint32_t logX, logY;
-        rays_per_warp( (uint64_t)p.width * p.height, logX, logY );
-        const uint64_t tiles = (uint64_t)( ( ( p.width - 1u ) >> logX ) + 1u ) * ( ( ( p.height - 1u ) >> logY ) + 1u );
+        const uint64_t pixels  = (uint64_t)p.width * p.height;
+        const bool     general = general_search( b, st, 0 );
         uint32_t *     list, *flags;
-        const SdfIndex ix = build_index( b, st, nullptr, 0, true, (uint64_t)p.width * p.height >= b.n, band, scratch, list, flags, s );
-        k_trace<<<(uint32_t)std::min<uint64_t>( blocks_of( tiles, kSdfWarps ), 152u * 64u ), 32 * kSdfWarps, 0, s>>>( b, ix, p, band, logX, logY, depth,
-                                                                                                                     normals );
+        const SdfIndex ix = build_index( b, st, nullptr, 0, !general, pixels >= b.n, band, scratch, list, flags, s );
+        if ( !general )
+        {
+            uint32_t logX, logY;
+            rays_per_warp( pixels, logX, logY );
+            const uint64_t tiles = (uint64_t)( ( ( p.width - 1u ) >> logX ) + 1u ) * ( ( ( p.height - 1u ) >> logY ) + 1u );
+            k_trace<true><<<(uint32_t)std::min<uint64_t>( blocks_of( tiles, kSdfWarps ), 152u * 64u ), 32 * kSdfWarps, 0, s>>>( b, ix, p, band, logX,
+                                                                                                                             logY, depth, normals );
+            count_launches( 1 );
+        }
+        k_trace<false><<<(uint32_t)std::min<uint64_t>( blocks_of( pixels, kSdfWarps ), 152u * 32u ), 32 * kSdfWarps, 0, s>>>( b, ix, p, band, 0, 0, depth,
+                                                                                                                           normals );
         count_launches( 1 );
     }
 

@@ -1,4 +1,4 @@
-"""Builds whose signed distance takes the general search alone: truncated neighbour lists, atoms outside the box,
+"""Builds whose signed distance and image take the general search alone: truncated neighbour lists, atoms outside the box,
 spheres of tens of A; and arcs in more pieces than their buffer holds, which only the device finds out. The values are
 those of the general search on the same molecule with an atom outside its box, and nothing is launched for tiles."""
 import numpy as np
@@ -9,6 +9,22 @@ from sesdf_gb300.api import aabb
 from test_gpu_sdf_tile import evaluate
 
 pytestmark = pytest.mark.gpu
+
+
+def camera(atoms, width, height):
+    lo, hi = atoms[:, :3].min(0), atoms[:, :3].max(0)
+    centre, rad = 0.5 * (lo + hi).astype(np.float64), 0.5 * float(np.linalg.norm(hi - lo)) + 30.0
+    return {"eye": centre + [0, -3.0 * rad, 0], "forward": [0, 1, 0], "right": [1, 0, 0], "up": [0, 0, 1], "tan_half_fov": 0.36,
+            "t_near": rad, "t_far": 5.0 * rad, "eps": 1e-3, "normal_step": 1e-2, "width": width, "height": height, "max_steps": 2000}
+
+
+def image(g, cam):
+    import torch
+    depth = torch.full((cam["height"], cam["width"]), -1.0, device="cuda")
+    normals = torch.full((cam["height"], cam["width"], 3), -1.0, device="cuda")
+    g.render(cam, depth.data_ptr(), normals.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return depth.cpu().numpy(), normals.cpu().numpy()
 
 
 def launches(call):
@@ -40,22 +56,25 @@ def test_values_are_those_of_the_general_search(name):
     d = rng.normal(size=(3000, 3))
     q = (atoms[k, :3] + d / np.linalg.norm(d, axis=1)[:, None] * (atoms[k, 3:] + rng.uniform(-0.9 * rp, 1.5, (3000, 1)))).astype(np.float32)
     gq = rng.standard_normal(len(q)).astype(np.float32)
+    cam = camera(atoms, 70, 50)
     out = []
     for box in (None, aabb(atoms)):
         with SesBuild(both, rp, "full", box=box, max_neighbor_per_atom=288) as g:
             g.build()
             assert g.counts()["outside_atoms"] == (box is not None) and g.counts()["truncated_atoms"] == 0
-            out.append(evaluate(g, q, gq))
-    (got, kind, grad), (want, wkind, wgrad) = out
+            out.append((evaluate(g, q, gq), image(g, cam)))
+    ((got, kind, grad), im), ((want, wkind, wgrad), wim) = out
     assert np.array_equal(got, want) and np.mean(kind == wkind) > 0.999
     assert len(np.unique(kind)) > 3
     assert np.linalg.norm(grad - wgrad) <= 1e-4 * np.linalg.norm(wgrad)
+    assert np.isfinite(im[0]).any() and np.array_equal(im[0], wim[0]) and np.array_equal(im[1], wim[1], equal_nan=True)
 
 
 def test_general_builds_launch_nothing_for_tiles():
-    # without truncated lists one kernel more, for the arcs
+    # without truncated lists one kernel more for the arcs, of queries and of an image, and one for the image's tiles
     import torch
     atoms = synth.globule(1500, 62)
+    cam = camera(atoms, 16, 16)
     q = torch.from_numpy(synth.queries(atoms, 1000, 3)).cuda()
     out, grad = torch.empty(1000, device="cuda"), torch.empty(1500, 4, device="cuda")
     counts = []
@@ -64,7 +83,8 @@ def test_general_builds_launch_nothing_for_tiles():
             g.build()
             assert (g.counts()["truncated_atoms"] > 0) == (slots == 16)
             counts.append([launches(lambda: g.sdf(q.data_ptr(), 1000, out.data_ptr())),
-                           launches(lambda: g.sdf_backward(q.data_ptr(), 1000, out.data_ptr(), grad.data_ptr()))])
+                           launches(lambda: g.sdf_backward(q.data_ptr(), 1000, out.data_ptr(), grad.data_ptr())),
+                           launches(lambda: image(g, cam))])
             torch.cuda.synchronize()
     # (the scan of the general search's fewer cells may be a launch shorter too)
-    assert all(t - g >= less for g, t, less in zip(*counts, (1, 1)))
+    assert all(t - g >= less for g, t, less in zip(*counts, (1, 1, 2)))
