@@ -7,14 +7,15 @@
 //   x inside the SAS:   sdf = rp - min(T, dist(x, dE)).
 // dE is the SAS surface: the accessible parts of the SAS spheres, the arcs of
 // the visible circles and the probe positions. The nearest point of dE is the
-// radial projection of x on a sphere, the nearest point of a circle, or a
-// probe, whichever is nearest among those that lie on dE (not strictly inside
-// another SAS sphere); only atoms with |x - c_i| <= R_i + T can carry one.
+// radial projection of x on a sphere, the nearest point of a circle (any one
+// where x lies on its axis), or a probe, whichever is nearest among those that
+// lie on dE (not strictly inside another SAS sphere); only atoms with
+// |x - c_i| <= R_i + T can carry one.
 // The gradient with respect to the atoms follows the active primitive: the
 // sphere or atom distance directly, a circle point and a probe by the
 // Lagrange / implicit-function rule for points constrained to |p - c_m| = R_m.
 //
-// Two searches give every value, the same to the last bit. The general search (sdf_query, a
+// Two searches give every value, the same to the last bit. The general search (sdf_query_pass, a
 // warp per query) examines the atoms within reach in the order of their lower bound, every
 // visible circle of each, with the accessibility of every candidate point settled in double
 // precision where float32 cannot. The tile search (sdf_tile_search, a lane per query or a
@@ -72,7 +73,8 @@ namespace sesgb
         }
 
         // Nearest point q of circle (i, j) to x and its distance; nj = (c_j, R_j). -1: no circle; 0: x on the
-        // axis (q the centre, dist that of any point); 1 otherwise.
+        // axis (q the centre, dist that of any point); 1: next to it, where the rounding of x - c turns q by more than
+        // hidden_band allows; 2 otherwise.
         __device__ __forceinline__ int sdf_circle_point( float3 x, float4 ci, float Ri, float4 nj, float & dist, float3 & q )
         {
             const float3 d  = make_float3( __fsub_rn( nj.x, ci.x ), __fsub_rn( nj.y, ci.y ), __fsub_rn( nj.z, ci.z ) );
@@ -98,7 +100,7 @@ namespace sesgb
             const float s = __fdiv_rn( r, rho ), e = __fsub_rn( rho, r );
             q             = make_float3( __fmaf_rn( v.x, s, c.x ), __fmaf_rn( v.y, s, c.y ), __fmaf_rn( v.z, s, c.z ) );
             dist          = __fsqrt_rn( __fmaf_rn( h, h, __fmul_rn( e, e ) ) );
-            return 1;
+            return rho > 0.02f ? 2 : 1;
         }
 
         constexpr int   kSdfWarps = 4;   // warps per block (one query per warp)
@@ -222,6 +224,58 @@ namespace sesgb
                     return true;
             }
             return false;
+        }
+
+        // A point of circle (i, neighbour slot s), all as far from x, lies in no SAS sphere of a near neighbour of i other than
+        // that of slot s: in double precision. An uncovered arc ends where a sphere meets the circle, in a point that no
+        // other one holds.
+        __device__ __noinline__ bool circle_open_d( const Build & b, const SdfSmem & sm, size_t row, uint32_t nn, uint32_t i, uint32_t s )
+        {
+            const float4 ai = b.atoms[ i ], aj = b.atoms[ b.nbr[ row + s ] ];
+            const double Ri = (double)ai.w + (double)b.rp, Rj = (double)aj.w + (double)b.rp;
+            const d3     d  = D3( (double)aj.x - (double)ai.x, (double)aj.y - (double)ai.y, (double)aj.z - (double)ai.z );
+            const double dd = ddot( d, d ), tt = ( Ri * Ri - Rj * Rj + dd ) / ( 2.0 * dd ), r2 = Ri * Ri - tt * tt * dd;
+            if ( !( r2 > 0.0 ) )
+                return true;
+            const double r = sqrt( r2 );
+            const d3     n = dmul( d, 1.0 / sqrt( dd ) ), c = dadd( D3( ai ), dmul( d, tt ) );
+            bool         cut = false;
+            for ( uint32_t e = 0; e < nn; e++ )
+            {
+                const uint32_t k = sm.near[ e ];
+                if ( k == s )
+                    continue;
+                // hidden where A + B cos(phi - phi_k) > 0, phi_k the direction v of c_k from the axis
+                const float4 ak = b.atoms[ b.nbr[ row + k ] ];
+                const double Rk = (double)ak.w + (double)b.rp;
+                const d3     w  = dsub( D3( ak ), c );
+                const double h  = ddot( w, n );
+                const d3     v  = dsub( w, dmul( n, h ) );
+                const double l = sqrt( ddot( v, v ) ), A = Rk * Rk - ddot( w, w ) - r2, B = 2.0 * r * l;
+                if ( A > B )
+                    return false;
+                if ( !( A > -B ) || !( l > 0.0 ) )
+                    continue;
+                cut            = true;
+                const double cs = -A / B, sn = sqrt( fmax( 0.0, ( 1.0 - cs ) * ( 1.0 + cs ) ) );
+                const d3     u = dmul( v, r * cs / l ), t = dmul( dcross( n, v ), r * sn / l );
+                for ( int side = 0; side < 2; side++ )
+                {
+                    const d3 q    = dadd( c, side ? dsub( u, t ) : dadd( u, t ) );
+                    bool     open = true;
+                    for ( uint32_t o = 0; o < nn && open; o++ )
+                    {
+                        const float4 ao = b.atoms[ b.nbr[ row + sm.near[ o ] ] ];
+                        const double Ro = (double)ao.w + (double)b.rp;
+                        const d3     y  = dsub( q, D3( ao ) );
+                        // (by more than rounding: spheres of a lattice meet in one point)
+                        open = o == e || sm.near[ o ] == s || !( ddot( y, y ) < Ro * Ro * ( 1.0 - 1e-11 ) );
+                    }
+                    if ( open )
+                        return true;
+                }
+            }
+            return !cut;
         }
 
         // The general search: one query, the whole warp; the hit is valid in every lane. A point of dE
@@ -485,8 +539,8 @@ namespace sesgb
                     {
                         if ( !( dist < cand ) || !( dist < best ) )
                             continue;
-                        bool hidden = false, unsure = false;
-                        for ( uint32_t e = 0; e < nn && !hidden; e++ )
+                        bool hidden = false, unsure = at == 1;
+                        for ( uint32_t e = 0; at > 1 && e < nn && !hidden; e++ )
                         {
                             const uint32_t k = sm.near[ e ];
                             if ( k == s )
@@ -511,10 +565,17 @@ namespace sesgb
                     }
                     else
                     {
-                        // x on the axis: every point of the circle is as near; a visible
-                        // circle has an accessible arc
+                        // x on the axis: every point of the circle is as near. A visible circle is one that no single
+                        // sphere buries; several together may
                         if ( !( dist < cand ) || !( dist < best ) )
                             continue;
+                        if constexpr ( kExact )
+                        {
+                            if ( !circle_open_d( b, sm, row, nn, i, s ) )
+                                continue;
+                        }
+                        else
+                            exactLane = true;
                     }
                     cand = dist;
                     ck   = kSdfCircle;
@@ -1032,7 +1093,6 @@ namespace sesgb
         // ---- tile search -----------------------------------------------------------------------
         constexpr int   kTileAtoms = 256;  // atoms around a tile
         constexpr int   kTileItems = 192;  // probes or arcs held at a time
-        constexpr float kAxisReach = 1.2f; // x is tried against the lines through centres within this (points on bonds)
         constexpr float kTileEdge  = 4.f;  // queries of one tile lie within this of its first one
 
         struct TileSmem
@@ -1653,7 +1713,6 @@ namespace sesgb
                         continue;
                     }
                 }
-                ByteQueue close { 0ull, 0 }; // atoms whose centre is next to x
                 for ( uint32_t w = 0; w * 32u < na; w++ )
                 {
                     uint32_t bits = 0;
@@ -1664,8 +1723,6 @@ namespace sesgb
                             const f3     v = F3( xr.x - p.x, xr.y - p.y, xr.z - p.z );
                             const float  r = cut + p.w, d = dot( v, v );
                             bits |= ( d < r * r ? 1u : 0u ) << ( k & 31u );
-                            if ( d < kAxisReach * kAxisReach && close.n < 8 )
-                                close.push( k );
                         }
                     for ( uint32_t o = 1; o < G; o <<= 1 )
                         bits |= __shfl_xor_sync( 0xffffffffu, bits, o );
@@ -1673,30 +1730,6 @@ namespace sesgb
                         sm.near[ w ][ query ] = bits;
                 }
                 __syncwarp();
-
-                // a point on a circle's axis is as near to all of it, and the general search takes a visible
-                // circle then without a look at its arcs: at a centre, or on the line of two centres
-                while ( __any_sync( 0xffffffffu, close.n > 0 ) )
-                {
-                    if ( close.n == 0 )
-                        continue;
-                    const float4 p = sm.atom[ close.pop() ];
-                    const f3     v = F3( xr.x - p.x, xr.y - p.y, xr.z - p.z );
-                    if ( dot( v, v ) < 1e-4f )
-                        exact = true;
-                    for ( uint32_t w = 0; w * 32u < na && !exact; w++ )
-                        for ( uint32_t bits = sm.near[ w ][ query ]; bits; bits &= bits - 1u )
-                        {
-                            const float4 o = sm.atom[ w * 32u + (uint32_t)__ffs( (int)bits ) - 1u ];
-                            const f3     u = F3( o.x - p.x, o.y - p.y, o.z - p.z );
-                            const f3     c = cross( v, u );
-                            const float  d = dot( u, u );
-                            if ( d > 0.f && dot( c, c ) < tol * tol * d )
-                                exact = true;
-                        }
-                }
-                for ( uint32_t o = 1; o < G; o <<= 1 )
-                    exact |= __shfl_xor_sync( 0xffffffffu, exact ? 1 : 0, o ) != 0;
 
                 // radial projections on the SAS spheres
                 {
