@@ -395,7 +395,8 @@ namespace sesgb
                             continue;
                         const float4 p    = b.stagePos[ chunk + e ];
                         const float  dist = sdf_distance( x, p );
-                        if ( dist < cand )
+                        // (of equal distances the lowest atom's, the first of its chunk: the list's order differs from call to call)
+                        if ( dist < cand || ( dist == cand && (int)i < pa ) )
                         {
                             const int4 ids = b.stageIds[ chunk + e ];
                             cand           = dist;
@@ -407,10 +408,13 @@ namespace sesgb
                     }
                 }
                 float wbest = cand;
-                int   owner = (int)lane;
-                warp_min_hit( wbest, owner );
+                for ( int o = 16; o > 0; o >>= 1 )
+                    wbest = fminf( wbest, __shfl_xor_sync( 0xffffffffu, wbest, o ) );
                 if ( wbest < best )
                 {
+                    const uint32_t key   = cand == wbest ? (uint32_t)pa : 0xffffffffu;
+                    const uint32_t first = __reduce_min_sync( 0xffffffffu, key );
+                    const int      owner = __ffs( (int)__ballot_sync( 0xffffffffu, key == first ) ) - 1;
                     best     = wbest;
                     hit.kind = kSdfProbe;
                     hit.a    = __shfl_sync( 0xffffffffu, pa, owner );
@@ -1243,6 +1247,17 @@ namespace sesgb
             return false;
         }
 
+        // probe p before probe q in the order of the general search: by their atoms, then as they were found
+        __device__ __noinline__ bool probe_before( const int4 * ids, int p, int q )
+        {
+            const int4 a = ids[ p ], c = ids[ q ];
+            if ( a.x != c.x )
+                return a.x < c.x;
+            if ( a.y != c.y )
+                return a.y < c.y;
+            return a.z != c.z ? a.z < c.z : p < q;
+        }
+
         // slot of target in an ascending neighbour row that holds it
         __device__ __forceinline__ uint32_t slot_of( const uint32_t * row, uint32_t len, uint32_t target )
         {
@@ -1672,7 +1687,7 @@ namespace sesgb
                             }
                     }
                     // the general search takes the nearest one, by its own distances where the screened ones do not
-                    // tell (a distance carries a few roundings of its own size only); of equal ones either
+                    // tell (a distance carries a few roundings of its own size only); of equal ones the first in its order
                     const float near = 5e-7f * ext;
                     float       dp   = p0 >= 0 ? sdf_distance( x, b.probePos[ p0 ] ) : inf;
                     if ( screen_sqrt( d1 ) <= dp + near )
@@ -1684,16 +1699,18 @@ namespace sesgb
                             if ( e )
                                 best.dropped = 0.f; // (a fourth one would not be seen)
                             const float d = sdf_distance( x, b.probePos[ q ] );
-                            p0            = d < dp ? q : p0;
-                            dp            = fminf( d, dp );
+                            if ( d < dp || ( d == dp && probe_before( b.probeIds, q, p0 ) ) )
+                                p0 = q;
+                            dp = fminf( d, dp );
                         }
                     for ( uint32_t o = 1; o < G; o <<= 1 )
                     {
                         const float d = __shfl_xor_sync( 0xffffffffu, dp, o );
                         const int   q = __shfl_xor_sync( 0xffffffffu, p0, o );
                         best.dropped  = fminf( best.dropped, __shfl_xor_sync( 0xffffffffu, best.dropped, o ) );
-                        p0            = d < dp || ( d == dp && q < p0 ) ? q : p0;
-                        dp            = fminf( d, dp );
+                        if ( d < dp || ( d == dp && q >= 0 && q != p0 && probe_before( b.probeIds, q, p0 ) ) )
+                            p0 = q;
+                        dp = fminf( d, dp );
                     }
                     if ( p0 >= 0 )
                         best.insert( { dp, kSdfProbe, p0, -1 }, tol );
