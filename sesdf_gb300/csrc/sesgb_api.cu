@@ -230,8 +230,9 @@ namespace
                                   &b.chunkLen, &b.pairOff };
             for ( uint32_t ** p : per )
                 *p = L.take<uint32_t>( n + 1 );
-            b.convex = L.take<uint2>( n );
-            b.counts = L.take<DeviceCounts>( 1 );
+            b.wideOff = L.take<uint32_t>( n );
+            b.convex  = L.take<uint2>( n );
+            b.counts  = L.take<DeviceCounts>( 1 );
             c->radixScratch = L.take<char>( radix_scratch_bytes( c->n ) );
         } );
         if ( !got || !cuda_ok( c, cudaMallocHost( &c->hCounts, sizeof( DeviceCounts ) ), "cudaMallocHost" ) )
@@ -284,7 +285,7 @@ namespace
             b.segments    = L.take<uint4>( b.capSeg );
             b.visBand     = L.take<uint2>( b.capVisBand );
             b.touch       = L.take<uint64_t>( b.capPairs );
-            b.touchHigh   = L.take<uint64_t>( b.capPairs );
+            b.touchHigh   = L.take<uint64_t>( b.capWide );
             b.torPos      = L.take<float4>( b.capTori );
             b.torAxis     = L.take<float4>( b.capTori );
             b.torVs       = L.take<float4>( b.capTori );
@@ -431,6 +432,7 @@ namespace
         b.capProbes        = grow( 8ull * n );
         b.capVisBand       = grow( n ? std::max<uint64_t>( 1u << 16, n / 2 ) : 0 );
         b.capPairs         = grow( 40ull * n );
+        b.capWide          = grow( ( c->rp > 1.5f ? 40ull : 4ull ) * n ); // lists beyond 64 are rare at 1.4 A
         b.capSeg           = grow( 8ull * n );
         b.capTori          = grow( 16ull * n );
     }
@@ -457,6 +459,7 @@ namespace
         fix( b.capTori, h.T );
         fix( b.capVisBand, h.visBand );
         fix( b.capPairs, h.P );
+        fix( b.capWide, h.wide );
         if ( h.overflow & ( kOverflowProbes | kOverflowList ) )
         {
             // sizes follow I; a list overflow means a circle with more probes than one
@@ -562,7 +565,7 @@ namespace
         const Build &        b = c->b;
         return ( h.overflow & ~(uint32_t)kOverflowNbr ) == 0 && h.V <= b.capSectors && h.F <= b.capFull && h.C1 <= b.capC1
                && h.staged <= b.capProbes && h.I <= b.capProbes && h.S <= b.capSeg && h.T <= b.capTori
-               && h.visBand <= b.capVisBand && h.P <= b.capPairs;
+               && h.visBand <= b.capVisBand && h.P <= b.capPairs && h.wide <= b.capWide;
     }
 
     // waits for the enqueued build; on a capacity overflow regrows and builds again

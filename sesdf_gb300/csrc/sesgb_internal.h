@@ -59,6 +59,7 @@ namespace sesgb
         uint32_t segCircles; // circles carrying at least two probes
         uint32_t visBand;    // visibility tests queued for double precision
         uint32_t probeCursor; // work counter of the persistent probe screen
+        uint32_t wide;        // neighbour pairs of the atoms with 65 to 128 neighbours
     };
     static_assert( offsetof( DeviceCounts, staged ) % 8 == 0 && offsetof( DeviceCounts, jobs ) == offsetof( DeviceCounts, staged ) + 4,
                    "staged and jobs form one 8-byte word" );

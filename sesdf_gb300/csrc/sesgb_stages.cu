@@ -644,6 +644,9 @@ namespace sesgb
             // operations.cu:126-204; the two differ only inside its float32 band)
             float    d2max = 0.f, r2max = 0.f;
             uint32_t nc    = 0;
+            // the high words of a wide atom's masks lie where it comes to take them
+            if ( lane == 0 && ni > (uint32_t)kMaskSlots && ni <= (uint32_t)kWideSlots )
+                b.wideOff[ i ] = atomicAdd( &b.counts->wide, ni );
             for ( uint32_t base = 0; base < ni + 32; base += 32 )
             {
                 const uint32_t s    = base + lane;
@@ -799,8 +802,9 @@ namespace sesgb
                         x = first == 0u || first >= 128u ? 0ull : first < 64u ? t >> ( 64u - first ) : t << ( first - 64u );
                         for ( uint32_t o = 1; o < G; o <<= 1 )
                             x |= __shfl_xor_sync( 0xffffffffu, x, o );
-                        if ( own && at < b.capPairs )
-                            b.touchHigh[ at ] = x;
+                        const uint32_t high = own ? b.wideOff[ i ] + s : 0u;
+                        if ( own && high < b.capWide )
+                            b.touchHigh[ high ] = x;
                     }
                 }
                 if ( valid && gl == 0 && ( gb || gt ) )
@@ -1378,7 +1382,7 @@ namespace sesgb
         // (both entries reserved for the double-precision pass).
         template<bool useMask>
         __device__ __forceinline__ void probe_screen( const ProbeSmem & m, const ProbeBounds & pb, float Ri, float rp,
-                                                      uint32_t ni, const Build & b, uint32_t po, bool wide,
+                                                      uint32_t ni, const Build & b, uint32_t po, uint32_t wo, bool wide,
                                                       uint32_t sj, uint32_t sk, int w[ 2 ], bool & band )
         {
             const float4 qj = m.rel[ sj ], qk = m.rel[ sk ];
@@ -1456,7 +1460,7 @@ namespace sesgb
                     uint32_t w = 0xffffffffu >> ( ni - base < 32u ? 32u - ( ni - base ) : 0u );
                     if ( wide )
                     {
-                        const uint64_t * t = ( base < 64u ? b.touch : b.touchHigh ) + po;
+                        const uint64_t * t = base < 64u ? b.touch + po : b.touchHigh + wo;
                         w &= (uint32_t)( ( t[ sj ] & t[ sk ] ) >> ( base & 32u ) );
                     }
                     if ( sj - base < 32u )
@@ -1503,7 +1507,8 @@ namespace sesgb
 
             // atoms of 65 to 128 neighbours (a larger probe radius): their masks stay in global memory. 6,007 atoms with a
             // 2.4 A probe: this kernel 183 -> 102 us against trying every neighbour (25 of 80 remain)
-            const bool wide    = !useMask && ni <= (uint32_t)kWideSlots && po + ni <= b.capPairs;
+            const uint32_t wo   = !useMask && ni <= (uint32_t)kWideSlots ? b.wideOff[ i ] : 0u;
+            const bool     wide = !useMask && ni <= (uint32_t)kWideSlots && po + ni <= b.capPairs && wo + ni <= b.capWide;
             uint32_t   p       = 0;
             uint64_t   partial = 0; // slots of the partial circles (i, j), i < j
             float      d2max = 0.f, bmax = 0.f;
@@ -1601,7 +1606,7 @@ namespace sesgb
                     if ( lane < batch )
                     {
                         sjk = m.cand[ lane ];
-                        probe_screen<useMask>( m, pb, Ri, b.rp, ni, b, po, wide, sjk & 0xffffu, sjk >> 16, w, band );
+                        probe_screen<useMask>( m, pb, Ri, b.rp, ni, b, po, wo, wide, sjk & 0xffffu, sjk >> 16, w, band );
                     }
                     const uint32_t need = band ? 2u : ( w[ 0 ] != 0 ) + ( w[ 1 ] != 0 );
                     uint32_t       tot;
@@ -1734,7 +1739,7 @@ namespace sesgb
                         if ( wide )
                         {
                             // the far atom has to touch circle (i, j)
-                            const bool far = isC && !( ( ( sk < 64u ? b.touch : b.touchHigh )[ po + sj ] >> ( sk & 63u ) ) & 1u );
+                            const bool far = isC && !( ( ( sk < 64u ? b.touch + po : b.touchHigh + wo )[ sj ] >> ( sk & 63u ) ) & 1u );
                             cands += __popc( __ballot_sync( 0xffffffffu, far ) );
                             isC = isC && !far;
                         }

@@ -69,8 +69,10 @@ namespace sesgb
         uint32_t   capVisBand;
         uint32_t * pairOff;  // n + 1: first pair of each atom (exclusive count of the neighbour lists)
         uint64_t * touch;    // capPairs, at pairOff[i] + s: neighbours that may hold a point of circle (i, s), slots 0 to 63
-        uint64_t * touchHigh; // slots 64 to 127 (atoms with more than 64 neighbours)
         uint32_t   capPairs;
+        uint64_t * touchHigh; // capWide, at wideOff[i] + s: slots 64 to 127 (atoms with 65 to 128 neighbours)
+        uint32_t * wideOff;   // n
+        uint32_t   capWide;
         uint32_t * slotTrim; // partial-circle number of each slot (exclusive count)
 
         // per-atom counts and offsets

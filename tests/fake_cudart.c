@@ -8,10 +8,12 @@
 static int          fail_mallocs, last_error;
 static unsigned     launches, mallocs, frees, poke_word, poke_value, poke_left;
 static const void * fill_from;
+static unsigned long long bytes;
 static size_t       fill_bytes;
 
 void     fake_fail( int n ) { fail_mallocs = n; }
 unsigned fake_launches( void ) { return launches; }
+unsigned long long fake_bytes( void ) { return bytes; } /* allocated so far */
 unsigned fake_live( void ) { return mallocs - frees; }
 /* the next `times` copies of a counter record (100 to 255 bytes) to the host have `value` in word `word` */
 void fake_poke( unsigned word, unsigned value, unsigned times )
@@ -36,6 +38,7 @@ int cudaMalloc( void ** p, size_t n )
         return last_error = 2; /* out of memory */
     }
     mallocs++;
+    bytes += n;
     *p = calloc( n ? n : 1, 1 );
     return 0;
 }

@@ -112,6 +112,20 @@ def cavity_buffers_fail(fake):
     assert fake.fake_live() == 0
 
 
-@pytest.mark.parametrize("body", ["regrow_fails", "query_buffers_fail", "cavity_buffers_fail"])
+def mask_bytes(fake):
+    # the masks of slots 64 to 127 have room for the atoms that such lists occur with: few at the usual probe radius
+    import numpy as np
+    from sesdf_gb300 import SesBuild
+    fake.fake_bytes.restype = ctypes.c_ulonglong
+    n, used = 100_000, []
+    atoms = np.random.default_rng(1).uniform(1, 100, (n, 4)).astype(np.float32)
+    for radius in (1.4, 2.4):
+        before = fake.fake_bytes()
+        SesBuild(atoms, radius, "full").close()
+        used.append(fake.fake_bytes() - before)
+    assert used[1] - used[0] >= 300 * n
+
+
+@pytest.mark.parametrize("body", ["mask_bytes", "regrow_fails", "query_buffers_fail", "cavity_buffers_fail"])
 def test_allocation_failure(shim, body):
     child(shim, body)
