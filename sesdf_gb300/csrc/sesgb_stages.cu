@@ -2537,9 +2537,10 @@ namespace sesgb
                 const float4   ai = b.atoms[ i ], aj = b.atoms[ j ];
 
                 const uint32_t st          = lst[ 0 ];
-                const int4     sids        = b.probeIds[ st ];
+                // (not .w, which k_probe_neighbors may be writing in the other branch of a recorded build)
+                const int *    sids        = &b.probeIds[ st ].x;
                 const float4   spos        = b.probePos[ st ];
-                const bool     isSecondary = (int)i == sids.x && (int)j == sids.z;
+                const bool     isSecondary = (int)i == sids[ 0 ] && (int)j == sids[ 2 ];
                 const bool     reverse     = ( spos.w < 0.f ) != isSecondary; // direction < 0
 
                 // float32 keys, coordinates relative to atom i. Two probes need none: the first
