@@ -2449,14 +2449,16 @@ namespace sesgb
 
         // Lanes per query. Few queries per atom make the tile of a warp wide, so that its lists are long, and few queries
         // leave the GPU idle; more lanes per query make the tile smaller and the walk over its lists shorter, and cost
-        // the tile's own work again. Measured over 2,000 to 100,000 atoms and 1,000 to 1,000,000 queries in the molecule's
+        // the tile's own work again. Measured over 2,000 to 100,000 atoms and 1,000 to 4,000,000 queries in the molecule's
         // box, the best G falls with m^(2/3) and grows with n^(1/3): 20,000 atoms with 20,000 queries 349 us at G = 16 (377
         // at 8, 353 at 32), with 200,000 queries 850 us at G = 4 (890 at 2, 939 at 8, 1123 at 1); 100,000 atoms with 200,000 queries
-        // 1867 us at 8 (2009 at 4, 1952 at 16). One lane from a million queries on: 2,000 atoms 1085 us at
-        // 1, 1145 at 2; 500,000 queries 805 and 612.
+        // 1867 us at 8 (2009 at 4, 1952 at 16). One lane and two (values / gradients, us): 2,000 atoms, 250,000 queries 531/573 and
+        // 525/633, 500,000 713/822 and 876/1063; 20,000 atoms, 1,000,000 queries 2536/2697 and 2280/2662, 1,500,000
+        // 3126/3376 and 3032/3603, 2,000,000 3563/3899 and 3818/4570; 100,000 atoms, 1,500,000 queries 5482/5767 and 5239/5938, 2,000,000
+        // 6199/6567 and 6119/7003.
         uint32_t lanes_per_query( uint32_t m, uint32_t n )
         {
-            uint32_t G = m < 1u << 20 ? 2u : 1u;
+            uint32_t G = m < std::min( 150000ull + 60ull * n, 1800000ull ) ? 2u : 1u;
             while ( G < 32u && (double)m * m * G * G * G < 3.2e7 * (double)n )
                 G *= 2u;
             return G;
