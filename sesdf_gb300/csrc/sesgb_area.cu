@@ -150,17 +150,6 @@ namespace sesgb
             return frame_angle( y1, t1 ) - frame_angle( y0, t0 );
         }
 
-        // atan2 to 1e-5 (Abramowitz and Stegun 4.4.49 on the smaller ratio), for bins with margins of 1e-3
-        __device__ __forceinline__ float bin_atan2( float y, float x )
-        {
-            const float ax = fabsf( x ), ay = fabsf( y );
-            const float z  = __fdividef( fminf( ax, ay ), fmaxf( fmaxf( ax, ay ), 1e-30f ) ), z2 = z * z;
-            float       a  = z * ( 0.9998660f + z2 * ( -0.3302995f + z2 * ( 0.1801410f + z2 * ( -0.0851330f + z2 * 0.0208351f ) ) ) );
-            a              = ay > ax ? 1.57079633f - a : a;
-            a              = x < 0.f ? 3.14159265f - a : a;
-            return copysignf( a, y );
-        }
-
         // A warp's work area for one region.
         struct RegionSmem
         {

@@ -125,7 +125,7 @@ namespace sesgb
 
         // A block takes 32 atoms: a thread per atom and axis finds the box of voxels in double precision, then a warp
         // takes an atom at a time. Bound by its atomics and the columns' float32 arithmetic. An FP64
-        // instruction occupies its pipe for 16 cycles whatever the lanes hold: with every column's run ends in
+        // instruction occupies its scheduler's pipe for 64 cycles whatever the lanes hold: with every column's run ends in
         // double precision, and every lane working out the box, 705 us for 20,000 atoms on a 0.5 A grid, 27 us now.
         __global__ void __launch_bounds__( 256 ) k_cav_raster( const float4 * atoms, uint32_t n, CavGrid g, double invh64, uint32_t * bits )
         {

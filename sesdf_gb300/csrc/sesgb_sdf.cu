@@ -745,17 +745,6 @@ namespace sesgb
             return normalize( v );
         }
 
-        // atan2 to 1e-5 (Abramowitz and Stegun 4.4.49 on the smaller ratio): the margins of the bins are 1e-3
-        __device__ __forceinline__ float bin_atan2( float y, float x )
-        {
-            const float ax = fabsf( x ), ay = fabsf( y );
-            const float z  = __fdividef( fminf( ax, ay ), fmaxf( fmaxf( ax, ay ), 1e-30f ) ), z2 = z * z;
-            float       a  = z * ( 0.9998660f + z2 * ( -0.3302995f + z2 * ( 0.1801410f + z2 * ( -0.0851330f + z2 * 0.0208351f ) ) ) );
-            a              = ay > ax ? 1.57079633f - a : a;
-            a              = x < 0.f ? 3.14159265f - a : a;
-            return copysignf( a, y );
-        }
-
         // What of every atom's SAS sphere and circles can be accessible. A warp per atom with an
         // accessible patch:
         //  - its directions in 256 bins, a lane per bin: the bins that no single neighbour's SAS sphere covers
