@@ -994,6 +994,7 @@ extern "C"
             return SESGB_ERR_INVALID;
         cudaStream_t s  = static_cast<cudaStream_t>( stream );
         SdfState     q;
+        q.pixels        = 0;
         int          st = sdf_prepare( c, m, q, s );
         if ( st != SESGB_OK )
             return st;
@@ -1008,6 +1009,7 @@ extern "C"
             return SESGB_ERR_INVALID;
         cudaStream_t s  = static_cast<cudaStream_t>( stream );
         SdfState     q;
+        q.pixels        = 0;
         int          st = sdf_prepare( c, m, q, s );
         if ( st != SESGB_OK )
             return st;
@@ -1025,6 +1027,7 @@ extern "C"
             return SESGB_ERR_INVALID;
         cudaStream_t s  = static_cast<cudaStream_t>( stream );
         SdfState     q;
+        q.pixels        = (uint64_t)cam->width * cam->height;
         int          st = sdf_prepare( c, 0, q, s );
         if ( st != SESGB_OK )
             return st;

@@ -295,6 +295,13 @@ namespace sesgb
             // outside the grid's box and sit in its border cells)
             const uint32_t total = stencil_rows_span2( ix.grid, ix.start, make_float4( x.x, x.y, x.z, 0.f ),
                                                        ix.outside ? 3e18f : ix.rmax + b.rp + T + 0.01f, sm.rowStart, sm.rowPre );
+            SdfHit hit;
+            hit.a = hit.b = hit.c = -1;
+            hit.q                 = x;
+            hit.kind              = kSdfClampOutside;
+            hit.value             = band;
+            if ( total == 0u )
+                return hit; // no atom near (most steps of most rays)
             // atoms within reach; minima of |x - c| - R (SAS) and |x - c| - r (vdW)
             uint32_t nl = 0;
             float    smin = 3.4e38f, vmin = 3.4e38f;
@@ -349,9 +356,6 @@ namespace sesgb
                     vatom = a;
                 }
             }
-            SdfHit hit;
-            hit.a = hit.b = hit.c = -1;
-            hit.q                 = x;
             if ( !( smin < 0.f ) )
             {
                 // outside the SAS (or nothing within reach)
@@ -360,11 +364,6 @@ namespace sesgb
                     hit.kind  = kSdfAtom;
                     hit.a     = vatom;
                     hit.value = vmin;
-                }
-                else
-                {
-                    hit.kind  = kSdfClampOutside;
-                    hit.value = band;
                 }
                 return hit;
             }
@@ -2473,10 +2472,16 @@ namespace sesgb
         // 20,000 queries 1522 and 2071, 26,000 2136 and 2146; 1,000,000 atoms, 100,000 queries 5579 and 7478, 150,000 8438 and
         // 8131. Uniform in the box the lines lie 10 to 20 % higher.
         bool general_only( uint32_t m, uint32_t n ) { return 12500ull * m <= n || 9ull * m + 55000u < n; }
-        // m: queries, 0 for an image
+        // Images of few pixels likewise: by the general search, a warp per ray, and by tiles 363 and 426 us for one pixel of 20,000
+        // atoms (1154 and 1026 for 8 x 8); 100,000 atoms, 64 x 64 pixels 2.79 and 3.12 ms, 128 x 128 7.0 and 5.2; 300,000 atoms,
+        // 128 x 128 6.5 and 7.8, 256 x 256 22.6 and 12.5; 1,000,000 atoms, 128 x 128 9.5 and 14.8, 256 x 256 34.0 and 23.9.
+        bool general_image( uint64_t pixels, uint32_t n )
+        {
+            return 12500ull * pixels <= n || ( 12ull * pixels + 50000u < n && pixels < 33000u );
+        }
         bool general_search( const Build & b, const SdfState & st, uint32_t m )
         {
-            return general_build( b, st ) || ( m && general_only( m, b.n ) );
+            return general_build( b, st ) || ( st.pixels ? general_image( st.pixels, b.n ) : general_only( m, b.n ) );
         }
 
         template<bool kBackward>
@@ -2526,7 +2531,7 @@ namespace sesgb
     {
         if ( !p.width || !p.height )
             return;
-        const uint64_t pixels  = (uint64_t)p.width * p.height;
+        const uint64_t pixels  = st.pixels;
         const bool     general = general_search( b, st, 0 );
         uint32_t *     list, *flags;
         const SdfIndex ix = build_index( b, st, nullptr, 0, !general, pixels >= b.n, band, scratch, list, flags, s );

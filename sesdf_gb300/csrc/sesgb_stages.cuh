@@ -146,6 +146,7 @@ namespace sesgb
         float rmax;      // largest vdW radius of the build
         bool  truncated; // neighbour lists
         bool  outside;   // atoms outside the grid's box
+        uint64_t pixels; // of an image; 0 for queries
     };
     size_t sdf_scratch_bytes( const Build & b, const SdfState & st, uint32_t m );
     void   launch_sdf( const Build & b, const SdfState & st, const float * queries, uint32_t m, float band, float * sdf, int * kind,

@@ -88,3 +88,24 @@ def test_general_builds_launch_nothing_for_tiles():
             torch.cuda.synchronize()
     # (the scan of the general search's fewer cells may be a launch shorter too)
     assert all(t - g >= less for g, t, less in zip(*counts, (1, 1, 2)))
+
+
+@pytest.mark.parametrize("n,few,many", [(12_500, (1, 1), (2, 1)), (65_000, (35, 35), (36, 35))])
+def test_images_of_few_pixels(n, few, many):
+    # either side of the number of pixels from which an image takes tiles: bits of the general search, and the kernels launched
+    atoms = synth.assembly(n // 2500, 2500)[: n - 1]
+    both = np.concatenate([atoms, np.float32([[*(atoms[:, :3].max(0) + 50.0), 1.5]])])
+    images, counts = [], []
+    for box in (None, aabb(atoms)):
+        with SesBuild(both, 1.4, "full", box=box) as g:
+            g.build()
+            for w, h in (few, many):
+                cam = camera(atoms, w, h)
+                if w < 3:  # at an atom
+                    cam.update(eye=atoms[0, :3] + [0, -3.0 * cam["t_near"], 0], tan_half_fov=1e-4)
+                image(g, cam)
+                counts.append(launches(lambda: images.append(image(g, cam))))
+    for k in range(2):
+        assert np.array_equal(images[k][0], images[2 + k][0]) and np.array_equal(images[k][1], images[2 + k][1], equal_nan=True)
+    assert np.isfinite(images[1][0]).any()
+    assert counts[0] <= counts[2] and counts[1] >= counts[3] + 2
