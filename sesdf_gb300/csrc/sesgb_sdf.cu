@@ -73,9 +73,9 @@ namespace sesgb
         }
 
         // Nearest point q of circle (i, j) to x and its distance; nj = (c_j, R_j). -1: no circle; 0: x on the
-        // axis (q the centre, dist that of any point); 1: next to it, where the rounding of x - c turns q by more than
-        // hidden_band allows; 2 otherwise.
-        __device__ __forceinline__ int sdf_circle_point( float3 x, float4 ci, float Ri, float4 nj, float & dist, float3 & q )
+        // axis (q the centre, dist that of any point); 1: next to it, where x - c hardly has a direction; 2 otherwise.
+        // turn: the radius over the distance of x from the axis, by which an error of x - c moves q.
+        __device__ __forceinline__ int sdf_circle_point( float3 x, float4 ci, float Ri, float4 nj, float & dist, float3 & q, float & turn )
         {
             const float3 d  = make_float3( __fsub_rn( nj.x, ci.x ), __fsub_rn( nj.y, ci.y ), __fsub_rn( nj.z, ci.z ) );
             const float  dd = sdf_dot( d, d ), Ri2 = __fmul_rn( Ri, Ri );
@@ -98,9 +98,10 @@ namespace sesgb
                 return 0;
             }
             const float s = __fdiv_rn( r, rho ), e = __fsub_rn( rho, r );
+            turn          = s;
             q             = make_float3( __fmaf_rn( v.x, s, c.x ), __fmaf_rn( v.y, s, c.y ), __fmaf_rn( v.z, s, c.z ) );
             dist          = __fsqrt_rn( __fmaf_rn( h, h, __fmul_rn( e, e ) ) );
-            return rho > 0.02f ? 2 : 1;
+            return rho > 1e-3f ? 2 : 1;
         }
 
         constexpr int   kSdfWarps = 4;   // warps per block (one query per warp)
@@ -533,16 +534,19 @@ namespace sesgb
                         if ( !( fabsf( Lj - nj.w ) < best ) )
                             continue;
                     }
-                    float        dist;
+                    float        dist, turn;
                     float3       q;
-                    const int    at = sdf_circle_point( x, ci, Ri, nj, dist, q );
+                    const int    at = sdf_circle_point( x, ci, Ri, nj, dist, q, turn );
                     if ( at < 0 )
                         continue;
                     if ( at > 0 )
                     {
                         if ( !( dist < cand ) || !( dist < best ) )
                             continue;
-                        bool hidden = false, unsure = at == 1;
+                        // x - c is off by up to 1.1e-7 coordinates + 1.2e-6, across the axis, and q by turn times that: 2 R_k times this is
+                        // 0.014 turn of hidden_band
+                        bool        hidden = false, unsure = at == 1;
+                        const float wide = 1.f + 0.03f * turn;
                         for ( uint32_t e = 0; at > 1 && e < nn && !hidden; e++ )
                         {
                             const uint32_t k = sm.near[ e ];
@@ -552,7 +556,7 @@ namespace sesgb
                             const float  dx = q.x - nk.x, dy = q.y - nk.y, dz = q.z - nk.z;
                             const float  d2 = dx * dx + dy * dy + dz * dz;
                             const float  m  = d2 - nk.w * nk.w;
-                            const float  eb = hidden_band( qQ, d2, nk.w );
+                            const float  eb = wide * hidden_band( qQ, d2, nk.w );
                             hidden          = m < -eb;
                             unsure          = unsure || !( fabsf( m ) > eb );
                         }
@@ -1308,8 +1312,9 @@ namespace sesgb
                     for ( int e = 0; e < 2; e++ )
                     {
                         const float4 u = e ? cj : ci, o = e ? ci : cj;
+                        float        turn;
                         const int    at =
-                            sdf_circle_point( x, u, u.w + b.rp, make_float4( o.x, o.y, o.z, o.w + b.rp ), dist[ events ], q[ events ] );
+                            sdf_circle_point( x, u, u.w + b.rp, make_float4( o.x, o.y, o.z, o.w + b.rp ), dist[ events ], q[ events ], turn );
                         if ( at == 0 )
                             return false;
                         if ( at < 0 )
@@ -1895,9 +1900,9 @@ namespace sesgb
                                     for ( int e = 0; e < 2; e++ )
                                     {
                                         const float4 u = e ? cj : ci, o = e ? ci : cj;
-                                        float        d;
+                                        float        d, turn;
                                         float3       t;
-                                        const int    at = sdf_circle_point( x, u, u.w + b.rp, make_float4( o.x, o.y, o.z, o.w + b.rp ), d, t );
+                                        const int    at = sdf_circle_point( x, u, u.w + b.rp, make_float4( o.x, o.y, o.z, o.w + b.rp ), d, t, turn );
                                         if ( at >= 0 )
                                             dm = fminf( dm, d );
                                         axis |= at == 0;
