@@ -2470,23 +2470,51 @@ namespace sesgb
             logY = pixels >= 3u << 16 ? 2u : pixels >= 3u << 11 ? 1u : 0u;
         }
 
-        // The general search alone, without arcs and tiles: one or a few queries, and few for the size of a large
-        // molecule, whose arcs cost 5.6 us per 1000 atoms whether or not a query comes near them. Queries near the
-        // surface, by the general search and by tiles: 20,000 atoms, 1 query 311 and 186 us (78 and 178 for one in the
-        // molecule's box), 2 queries 349 and 183; 100,000 atoms, 5000 queries 634 and 705, 7000 746 and 725; 300,000 atoms,
-        // 20,000 queries 1522 and 2071, 26,000 2136 and 2146; 1,000,000 atoms, 100,000 queries 5579 and 7478, 150,000 8438 and
-        // 8131. Uniform in the box the lines lie 10 to 20 % higher.
-        bool general_only( uint32_t m, uint32_t n ) { return 12500ull * m <= n || 9ull * m + 55000u < n; }
-        // Images of few pixels likewise: by the general search, a warp per ray, and by tiles 363 and 426 us for one pixel of 20,000
-        // atoms (1154 and 1026 for 8 x 8); 100,000 atoms, 64 x 64 pixels 2.79 and 3.12 ms, 128 x 128 7.0 and 5.2; 300,000 atoms,
-        // 128 x 128 6.5 and 7.8, 256 x 256 22.6 and 12.5; 1,000,000 atoms, 128 x 128 9.5 and 14.8, 256 x 256 34.0 and 23.9.
-        bool general_image( uint64_t pixels, uint32_t n )
+        // Whether the general search alone, without arcs and tiles, is the faster one. Before its first query the tile
+        // search finds the arcs of all atoms and bins these and the probes, 5.6 us per 1000 atoms; of the general
+        // search, the latency and the time per query grow with the atoms within reach and their neighbours, that is with a
+        // high power of the SAS radius R (of the largest atom; 3.2 A for a protein and a 1.4 A probe). In atoms' worth of arcs the latency is
+        // `lat`, a query `per`; a molecule of a few atoms is cheap to search at any radius. Measured over 1 to 1,000,000 atoms, probes of 0.4 to 2.8 A
+        // and 1 to 300,000 queries near the surface (general search and tiles, us):
+        //   1.4 A:  20,000 atoms, 1 query 311 and 186 (78 and 178 in the molecule's box), 2 queries 349 and 183; 100,000 atoms, 5000 queries
+        //           634 and 705, 7000 746 and 725; 300,000 atoms, 20,000 queries 1522 and 2071, 26,000 2136 and 2146;
+        //           1,000,000 atoms, 100,000 queries 5579 and 7478, 150,000 8438 and 8131
+        //   0.4 A:  tiles / general 1.07 and 0.81 for 5000 and 20,000 queries of 1000 atoms, 1.29 and 0.68 for 80,000 and 300,000 of 20,000
+        //   0.7 A:  1.06 and 0.79 for 20,000 and 80,000 queries of 20,000 atoms, 1.19 and 0.79 for 80,000 and 300,000 of 60,000
+        //   1.0 A:  1.27 and 0.96 for 64 and 300 queries of 20,000 atoms, 1.25 and 0.95 for 5000 and 20,000 of 60,000
+        //   2.0 A:  1.25 and 0.51 for 5000 and 20,000 queries of 200,000 atoms; 2.8 A: 1.05 and 0.80 for 1200 and 5000
+        //   10 atoms (any probe): 1.0 to 1.5 and 0.6 to 0.8 for 1200 and 20,000 queries; 1 atom 1.1 to 1.2 and 0.8 for 20,000 and 80,000
+        struct SearchCost
         {
-            return 12500ull * pixels <= n || ( 12ull * pixels + 50000u < n && pixels < 33000u );
+            double per, lat;
+            bool   cheap; // few atoms within reach of anything
+        };
+        SearchCost search_cost( float R, uint32_t n )
+        {
+            const double e = std::pow( std::max( 0.0, (double)R - 2.2 ), 1.5 );
+            return { std::pow( (double)R / 3.2, R < 3.2f ? 10.8 : 4.2 ), e, n <= 10u || n * e <= 25.0 };
+        }
+        bool general_only( uint32_t m, uint32_t n, float R )
+        {
+            const SearchCost c = search_cost( R, n );
+            return 12500ull * m <= n || 8.0 * c.per * m + 55000.0 * c.lat < n || ( c.cheap && m * std::pow( (double)n, 0.6 ) <= 20000.0 );
+        }
+        // Images of few pixels likewise: by the general search, a warp per ray, and by tiles (1.4 A) 363 and 426 us for one pixel of 20,000
+        // atoms (1154 and 1026 for 8 x 8); 100,000 atoms, 64 x 64 pixels 2.79 and 3.12 ms, 128 x 128 7.0 and 5.2; 300,000 atoms,
+        // 128 x 128 6.5 and 7.8, 256 x 256 22.6 and 12.5; 1,000,000 atoms, 128 x 128 9.5 and 14.8, 256 x 256 34.0 and 23.9. Cheap searches:
+        // tiles / general with a 0.4 A probe 1.1 to 1.5 at 256 x 256 pixels and 0.7 to 0.9 at 512 x 512 (300 to 20,000 atoms), with 0.7 A 1.0 to 1.2
+        // and 0.6 to 0.9; 1 atom 1.1 to 2.2 and 0.5 to 0.7.
+        bool general_image( uint64_t pixels, uint32_t n, float R )
+        {
+            const SearchCost c = search_cost( R, n );
+            const double     per = R < 3.2f ? c.per : c.per * c.per;
+            return 12500ull * pixels <= n || ( 12.0 * per * pixels + 50000.0 * c.lat < n && pixels < 33000u )
+                   || ( ( c.cheap || ( R < 2.55f && n <= 30000u ) ) && pixels <= 70000u );
         }
         bool general_search( const Build & b, const SdfState & st, uint32_t m )
         {
-            return general_build( b, st ) || ( st.pixels ? general_image( st.pixels, b.n ) : general_only( m, b.n ) );
+            const float R = st.rmax + b.rp;
+            return general_build( b, st ) || ( st.pixels ? general_image( st.pixels, b.n, R ) : general_only( m, b.n, R ) );
         }
 
         template<bool kBackward>

@@ -4,6 +4,7 @@ those of the general search on the same molecule with an atom outside its box, a
 import numpy as np
 import pytest
 
+from cases import hand_cases
 from sesdf_gb300 import SesBuild, api, synth
 from sesdf_gb300.api import aabb
 from test_gpu_sdf_tile import evaluate
@@ -109,3 +110,25 @@ def test_images_of_few_pixels(n, few, many):
         assert np.array_equal(images[k][0], images[2 + k][0]) and np.array_equal(images[k][1], images[2 + k][1], equal_nan=True)
     assert np.isfinite(images[1][0]).any()
     assert counts[0] <= counts[2] and counts[1] >= counts[3] + 2
+
+
+@pytest.mark.parametrize("name", ["single", "pair", "triangle", "collinear", "octahedron", "stack", "tangent"])
+def test_tiles_of_a_few_atoms(name):
+    # so many queries and pixels that molecules of a few atoms take tiles too: bits of the general search
+    atoms = hand_cases()[name]
+    both = np.concatenate([atoms, np.float32([[200.0, 0.0, 0.0, 1.5]])])
+    rng = np.random.default_rng(11)
+    m = 30_000
+    k = rng.integers(0, len(atoms), m)
+    q = (atoms[k, :3] + rng.normal(size=(m, 3)) * 2.0).astype(np.float32)
+    q[:2000:7] = atoms[k[:2000:7], :3]
+    q[1:2000:7] = 0.5 * (atoms[k[1:2000:7], :3] + atoms[k[2:2001:7], :3])
+    cam = camera(atoms, 270, 270)
+    out = []
+    for box in (None, aabb(atoms)):
+        with SesBuild(both, 1.4, "full", box=box) as g:
+            g.build()
+            out.append((evaluate(g, q), image(g, cam)))
+    ((got, kind, _), im), ((want, wkind, _), wim) = out
+    assert np.array_equal(got, want) and np.mean(kind == wkind) > 0.999
+    assert np.array_equal(im[0], wim[0]) and np.array_equal(im[1], wim[1], equal_nan=True)
