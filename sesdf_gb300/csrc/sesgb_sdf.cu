@@ -164,9 +164,10 @@ namespace sesgb
         // plus its reach) on every coordinate, times 2 |q - c_k| (taken as R_k: the bound matters only
         // where |q - c_k| is close to R_k), plus the rounding of the squares. Inside it the test is
         // taken again in double precision.
-        __device__ __forceinline__ float hidden_band( float qQ, float d2, float Rk )
+        constexpr float kHiddenBand = 3.8147e-6f;
+        __device__ __forceinline__ float hidden_band( float qQ, float d2, float Rk, float scale = kHiddenBand )
         {
-            return 3.8147e-6f * ( d2 + Rk * ( Rk + qQ ) + 1.f );
+            return scale * ( d2 + Rk * ( Rk + qQ ) + 1.f );
         }
 
         // point q (double) strictly inside the SAS sphere of atom k, in double precision
@@ -546,7 +547,7 @@ namespace sesgb
                         // x - c is off by up to 1.1e-7 coordinates + 1.2e-6, across the axis, and q by turn times that: 2 R_k times this is
                         // 0.014 turn of hidden_band
                         bool        hidden = false, unsure = at == 1;
-                        const float wide = 1.f + 0.03f * turn;
+                        const float wide = kHiddenBand * ( 1.f + 0.03f * turn );
                         for ( uint32_t e = 0; at > 1 && e < nn && !hidden; e++ )
                         {
                             const uint32_t k = sm.near[ e ];
@@ -556,7 +557,7 @@ namespace sesgb
                             const float  dx = q.x - nk.x, dy = q.y - nk.y, dz = q.z - nk.z;
                             const float  d2 = dx * dx + dy * dy + dz * dz;
                             const float  m  = d2 - nk.w * nk.w;
-                            const float  eb = wide * hidden_band( qQ, d2, nk.w );
+                            const float  eb = hidden_band( qQ, d2, nk.w, wide );
                             hidden          = m < -eb;
                             unsure          = unsure || !( fabsf( m ) > eb );
                         }
@@ -1962,10 +1963,10 @@ namespace sesgb
         static_assert( 32 * sizeof( TileHit ) <= sizeof( TileSmem ), "a warp's hits in its tile's memory" );
 
         // Queries in cell order, G lanes each (32 / G to a warp's tile); a query left to the general
-        // search goes to the list (one in 100,000). Issue- and latency-bound: 29,000 warp instructions a
-        // tile of 32 at 20 of 32 lanes, where the general search took 33,000 a query at 15. 1M queries around a
-        // 20,000-atom globule: 39.4 ms with the general search alone, 2.6 ms with this (2.0 ms here, 0.17 the
-        // arcs); 4,999 around 2,000 atoms: 483 and 119 us.
+        // search goes to the list (one in 100,000). Issue- and latency-bound: 15,000 warp instructions a
+        // tile of 16 (G = 2) at 22 of 32 lanes, where the general search takes 33,000 a query at 15. 1M queries around a
+        // 20,000-atom globule: 38.7 ms with the general search alone, 2.3 ms with this (1.96 ms here, 0.17 the
+        // arcs); 4,999 around 2,000 atoms: 489 and 115 us.
         template<bool kBackward>
         __global__ void __launch_bounds__( 32 * kSdfWarps ) k_sdf_tile( Build b, SdfIndex ix, const float * queries, uint32_t m, float band,
                                                                         uint32_t G, float * sdf, const float * gradSdf, float * gradSorted,
@@ -2037,7 +2038,7 @@ namespace sesgb
         // All m queries by the general search, a warp each, in cell order: the float32 pass; what it leaves open goes
         // to the list. Nothing here calls a function with the build (but for a gradient), and the pass fits 64 registers: eight blocks
         // a SM. Issue-bound (51 % at 15 of 32 lanes). 200,000 queries of 20,001 atoms one of which lies outside the box: 17.7 ms
-        // with both passes in one function at six blocks, 9.9 now; 1M atoms, 40,000 queries 3.75 and 2.9 ms.
+        // with both passes in one function at six blocks, 10.1 now; 1M atoms, 40,000 queries 3.75 and 2.9 ms.
         template<bool kBackward>
         __global__ void __launch_bounds__( 32 * kSdfWarps, 8 ) k_sdf_general( const __grid_constant__ Build b, const __grid_constant__ SdfIndex ix,
                                                                               const float * queries, uint32_t m, float band, float * sdf,
@@ -2140,7 +2141,7 @@ namespace sesgb
         // A warp takes 8 x 4 pixels or fewer (rays_per_warp), a lane each: their rays run close together, so that one tile
         // search serves the warp's points; the few points it leaves go through the general search one
         // after another. Bound by the longest rays: up to maxSteps searches one after another (512 x 512
-        // pixels of a 20,000-atom globule: 28.9 ms with a warp and a general search a ray, 13.2 ms).
+        // pixels of a 20,000-atom globule: 27.9 ms with a warp and a general search a ray, 12.9 ms).
         // kTiles false: the general search alone, a warp per ray.
         template<bool kTiles>
         __global__ void __launch_bounds__( 32 * kSdfWarps, kTiles ? 4 : 6 ) k_trace( const __grid_constant__ Build b, const __grid_constant__ SdfIndex ix,
@@ -2320,17 +2321,33 @@ namespace sesgb
         // arc pieces held: a protein has ~5 an atom; where more exist every query takes the general search
         uint32_t arc_capacity( uint32_t n ) { return 16u * n + 4096u; }
 
+        // Builds whose queries all take the general search: truncated neighbour lists, atoms outside the box, and
+        // SAS spheres or coordinates so large that the ball of an arc piece can pass kArcBall (k_sdf_arcs: half a piece is at most
+        // kArcHalf long, or half a bin of the largest circle).
+        bool general_build( const Build & b, const SdfState & st )
+        {
+            const float R    = st.rmax + b.rp;
+            const float half = std::max( kArcHalf + 1.1e-3f * R, R * std::sin( 0.5f * kArcStep + 1e-3f ) );
+            float       far  = 0.f;
+            for ( int a = 0; a < 3; a++ )
+            {
+                const float lo = ( &b.grid.origin.x )[ a ], hi = lo + ( &b.grid.cell.x )[ a ] * (float)b.grid.size;
+                far            = std::max( far, std::max( std::fabs( lo ), std::fabs( hi ) ) );
+            }
+            return st.truncated || st.outside || !( half + 1e-3f + 1e-6f * far < kArcBall );
+        }
+
         // Cells of half a query's reach over the reference grid's box, coarsened until they fit
-        // (a sparse molecule). For the general search alone 0.7 of it: fewer cells to zero and to scan, where few queries
-        // meet a large molecule (1,000 of 1M atoms 729 us with a half, 678 with 0.7, 716 with 1.0), and no slower
-        // elsewhere, as the rows of cells are cut to the reach; with atoms outside the box they are not.
+        // (a sparse molecule). For few queries of a large molecule, which take the general search, 0.7 of it: fewer cells to zero
+        // and to scan (1,000 queries of 1M atoms 729 us with a half, 678 with 0.7, 716 with 1.0); where all of a build's queries take it
+        // the half is faster (100,000 of 20,001 atoms 5458 us, 5618 with 0.7).
         void index_grid( const Build & b, const SdfState & st, float band, uint32_t m, uint32_t items, FineGrid & g, uint32_t & sub )
         {
             const double   size = b.grid.size;
             const double   e[ 3 ] = { b.grid.cell.x * size, b.grid.cell.y * size, b.grid.cell.z * size };
             const uint64_t most = std::min<uint64_t>( std::max<uint64_t>( 1u << 18, 24ull * b.n + 4ull * m ), 1u << 28 );
             sub                 = m ? 8u : 0u;
-            double h            = ( items == 1u && !st.outside ? 0.7 : 0.5 ) * ( st.rmax + 2.0 * b.rp + band );
+            double h            = ( items == 1u && !general_build( b, st ) ? 0.7 : 0.5 ) * ( st.rmax + 2.0 * b.rp + band );
             int    d[ 3 ]       = { 1, 1, 1 };
             for ( int it = 0; it < 400; it++ )
             {
@@ -2424,22 +2441,6 @@ namespace sesgb
             return ix;
         }
 
-        // Builds whose queries all take the general search: truncated neighbour lists, atoms outside the box, and
-        // SAS spheres or coordinates so large that the ball of an arc piece can pass kArcBall (k_sdf_arcs: half a piece is at most
-        // kArcHalf long, or half a bin of the largest circle).
-        bool general_build( const Build & b, const SdfState & st )
-        {
-            const float R    = st.rmax + b.rp;
-            const float half = std::max( kArcHalf + 1.1e-3f * R, R * std::sin( 0.5f * kArcStep + 1e-3f ) );
-            float       far  = 0.f;
-            for ( int a = 0; a < 3; a++ )
-            {
-                const float lo = ( &b.grid.origin.x )[ a ], hi = lo + ( &b.grid.cell.x )[ a ] * (float)b.grid.size;
-                far            = std::max( far, std::max( std::fabs( lo ), std::fabs( hi ) ) );
-            }
-            return st.truncated || st.outside || !( half + 1e-3f + 1e-6f * far < kArcBall );
-        }
-
         // Lanes per query. Few queries per atom make the tile of a warp wide, so that its lists are long, and few queries
         // leave the GPU idle; more lanes per query make the tile smaller and the walk over its lists shorter, and cost
         // the tile's own work again. Measured over 2,000 to 100,000 atoms and 1,000 to 4,000,000 queries in the molecule's
@@ -2526,9 +2527,10 @@ namespace sesgb
             if ( general_search( b, st, m ) )
             {
                 const SdfIndex ix = build_index( b, st, queries, m, false, false, band, scratch, list, flags, s );
-                // (more blocks than that would each wait for the longest of its queries: 1M atoms, 100,000 queries 5838 us, 5579 with
-                // warps that go on by themselves; few of these would leave SMs without work at the end)
-                k_sdf_general<kBackward><<<std::min( blocks_of( m, kSdfWarps ), 152u * 32u ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, sdf, gradSdf, gradSorted, kind,
+                // Few queries of a large molecule by warps that go on by themselves (1M atoms, 100,000 queries 5838 us with blocks of four
+                // that each wait for the longest, 5579 so); other builds by the blocks (20,000 atoms, 2.9 A probe, 100,000 queries 61.0 and 57.2 ms).
+                const uint32_t most = general_build( b, st ) ? 0xffffffffu : 152u * 32u;
+                k_sdf_general<kBackward><<<std::min( blocks_of( m, kSdfWarps ), most ), 32 * kSdfWarps, 0, s>>>( b, ix, queries, m, band, sdf, gradSdf, gradSorted, kind,
                                                                                               list, flags + 1 );
                 k_sdf_exact<kBackward><<<exactBlocks, 32 * kSdfWarps, 0, s>>>( b, ix, queries, band, sdf, gradSdf, gradSorted, kind, list, flags + 1 );
                 count_launches( 2 );
