@@ -186,7 +186,8 @@ int sesgb_build_device( sesgb_ctx * ctx, const void * device_atoms, void * strea
  * build on `stream` (device_atoms NULL = upload the borrowed host atoms) and
  * returns; sesgb_finish waits for it, and if a count exceeded a buffer's
  * capacity, regrows the buffer and builds again before returning. Results are
- * valid after sesgb_finish. */
+ * valid after sesgb_finish. Without the memory for a larger buffer a build
+ * returns SESGB_ERR_CUDA and leaves no results; the next one asks for it again. */
 int sesgb_build_async( sesgb_ctx * ctx, const void * device_atoms, void * stream );
 int sesgb_finish( sesgb_ctx * ctx );
 
