@@ -1240,10 +1240,16 @@ namespace sesgb
             return false;
         }
 
-        // probe p before probe q in the order of the general search: by their atoms, then as they were found
-        __device__ __noinline__ bool probe_before( const int4 * ids, int p, int q )
+        // Of probes p and q at the same float32 distance from x, whether p is taken: where they are as far in double precision too
+        // (by symmetry), by their atoms, then as they were found, as the general search does; else p if `lower`.
+        __device__ __noinline__ bool probe_first( const Build & b, float3 x, int p, int q, bool lower )
         {
-            const int4 a = ids[ p ], c = ids[ q ];
+            const d3     xd = D3( (double)x.x, (double)x.y, (double)x.z );
+            const d3     u = dsub( D3( b.probePos[ p ] ), xd ), v = dsub( D3( b.probePos[ q ] ), xd );
+            const double du = ddot( u, u ), dv = ddot( v, v );
+            if ( fabs( du - dv ) > 1e-12 * du )
+                return lower;
+            const int4 a = b.probeIds[ p ], c = b.probeIds[ q ];
             if ( a.x != c.x )
                 return a.x < c.x;
             if ( a.y != c.y )
@@ -1681,7 +1687,7 @@ namespace sesgb
                             }
                     }
                     // the general search takes the nearest one, by its own distances where the screened ones do not
-                    // tell (a distance carries a few roundings of its own size only); of equal ones the first in its order
+                    // tell (a distance carries a few roundings of its own size only); of equal ones as probe_first says
                     const float near = 5e-7f * ext;
                     float       dp   = p0 >= 0 ? sdf_distance( x, b.probePos[ p0 ] ) : inf;
                     if ( screen_sqrt( d1 ) <= dp + near )
@@ -1693,7 +1699,7 @@ namespace sesgb
                             if ( e )
                                 best.dropped = 0.f; // (a fourth one would not be seen)
                             const float d = sdf_distance( x, b.probePos[ q ] );
-                            if ( d < dp || ( d == dp && probe_before( b.probeIds, q, p0 ) ) )
+                            if ( d < dp || ( d == dp && probe_first( b, x, q, p0, false ) ) )
                                 p0 = q;
                             dp = fminf( d, dp );
                         }
@@ -1702,7 +1708,7 @@ namespace sesgb
                         const float d = __shfl_xor_sync( 0xffffffffu, dp, o );
                         const int   q = __shfl_xor_sync( 0xffffffffu, p0, o );
                         best.dropped  = fminf( best.dropped, __shfl_xor_sync( 0xffffffffu, best.dropped, o ) );
-                        if ( d < dp || ( d == dp && q >= 0 && q != p0 && probe_before( b.probeIds, q, p0 ) ) )
+                        if ( d < dp || ( d == dp && q >= 0 && q != p0 && probe_first( b, x, q, p0, q < p0 ) ) )
                             p0 = q;
                         dp = fminf( d, dp );
                     }
